@@ -60,7 +60,8 @@ typedef enum {
 
 typedef enum {
   WF_KERNEL_AUTO = 0,  /* fused when the grid allows it, else split          */
-  WF_KERNEL_FUSED = 1, /* one TMA z-march kernel per step (zero boundaries)  */
+  WF_KERNEL_FUSED = 1, /* H and E in one pass (zero boundaries): bricks or a
+                          TMA z-march                                       */
   WF_KERNEL_SPLIT = 2  /* an H kernel then an E kernel (any boundaries)      */
 } wf_kernel;
 
@@ -303,6 +304,10 @@ int64_t wf_kernel_launches(const wf_handle *h);
 
 /* ---- fused-kernel tiling (autotuner surface) --------------------------- */
 
+/* {8, 4, 1} names the brick step (one CTA per 32 x 8 x 4 cells, any boundary
+ * and CPML depth with FP32 storage); every other tiling is a z-march over
+ * 128-cell wide tiles.  By default the cheaper of the two for the grid's size
+ * and CPML runs; the results are bit-identical. */
 typedef struct {
   int32_t tile_rows;  /* y rows per CTA tile (x width is fixed at 128)      */
   int32_t z_chunk;    /* planes per CTA z-march                            */
@@ -320,6 +325,8 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms);
  * 128-cell tiles cover x in [16, nx-16) with no x-psi work; this applies when
  * the x CPML is at most 16 cells deep and nx >= 48.  Off: the wide tiles
  * cover the whole x range and their edge lanes run the x-psi recursion.
+ * Either call selects the z-march over the brick step, which has no column
+ * tiles, unless a tiling was set.
  * Results are bit-identical either way. */
 wf_status wf_set_column_tiles(wf_handle *h, int enable);
 /* 1 when the handle's fused step uses column tiles, 0 otherwise, -1 on a

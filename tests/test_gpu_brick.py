@@ -1,0 +1,106 @@
+"""GPU: the brick step against the split and marching kernels, bit for bit, at
+the sizes where it can go wrong: x extents that leave a brick 8, 16 or 24
+cells wide, single bricks, CPML depths that are not multiples of 4 (groups
+that straddle the slab), that meet in the middle or exceed 64 positions,
+periodic axes with and without CPML, more than 32 sources, sheet sources."""
+import numpy as np
+import pytest
+
+import wavefront_b200 as wf
+from wavefront_b200 import configs
+
+pytestmark = pytest.mark.gpu
+
+BRICK = (8, 4, 1)
+
+
+def _grid(dims, kernel, seed, pml=(0, 0, 0), periodic="", arith="exact", precision="f32",
+          tiling=None, nsrc=2, sheet=False, steps=9):
+    nx, ny, nz = dims
+    rng = np.random.default_rng(seed)
+    d = wf.GridDims(nx, ny, nz)
+    dx = 1e-3
+    dt = configs.courant_dt(dx)
+    g = wf.DeviceFieldGrid(d, kernel=kernel, arith=arith, precision=precision,
+                           boundary=tuple("periodic" if a in periodic else "zero" for a in "xyz"))
+    ids = rng.integers(0, 3, nx * ny * nz).astype(np.uint8)
+    table = wf.MaterialTable.vacuum_filled(dt, dx)
+    table.set_material(1, 4.0, 1.0, 0.01, dt, dx)
+    table.set_material(2, 2.25, 1.5, 0.0, dt, dx)
+    g.set_materials(wf.MaterialGrid(d, ids), table)
+    for ax, t in enumerate(pml):
+        if t:
+            p = wf.PmlProfile1D.build(dims[ax], wf.PmlConfig(thickness=t), dt, dx, t)
+            g.set_pml_axis(ax, t, p.b, p.a, p.inv_kappa)
+    if tiling:
+        g.set_tiling(*tiling)
+    f = rng.standard_normal((6, nz, ny, nx)).astype(np.float32)
+    f[3:] /= 377.0
+    g.set_fields(f)
+    if sheet:
+        g.add_source_values(nx - 1, 0, 0, 2, np.linspace(0.5, 1.0, steps), mode=1)
+    for k in range(nsrc):
+        # two share a cell: list order matters
+        x, y, z = (int(v) for v in (rng.integers(0, nx), rng.integers(0, ny), rng.integers(0, nz)))
+        for c in ([0, 0] if k == 0 else [k % 3]):
+            g.add_source_values(x, y, z, c, rng.standard_normal(steps).astype(np.float32))
+    for c in range(6):
+        tab = rng.standard_normal((steps, 2))
+        g.add_probe_tables(int(rng.integers(0, nx)), int(rng.integers(0, ny)), int(rng.integers(0, nz)), c,
+                           tab, tab + 1.0, 2, True)
+    g.step(steps)
+    g.sync()
+    out = [g.fields()] + [g.psi(w) for w in range(12)]
+    for c in range(6):
+        s = g.probe_sums(c, 2)
+        out += [s[0], s[1], np.array(s[2]), g.probe_trace(c, steps)]
+    g.close()
+    return out
+
+
+def _same(a, b):
+    for i, (u, v) in enumerate(zip(a, b)):
+        assert np.array_equal(u, v), f"output {i}: {int((u != v).sum())} values differ"  # +0 == -0
+
+
+@pytest.mark.parametrize("dims,pml,periodic,kw", [
+    ((8, 8, 8), (0, 0, 0), "", {}),
+    ((8, 8, 8), (4, 3, 4), "", {}),
+    ((40, 16, 8), (10, 5, 2), "", {}),
+    ((48, 8, 24), (24, 4, 1), "", {"nsrc": 33}),
+    ((56, 72, 16), (7, 16, 8), "", {"arith": "fma"}),
+    ((72, 16, 16), (36, 8, 8), "", {}),
+    ((160, 16, 16), (40, 0, 0), "", {}),
+    ((32, 24, 24), (0, 0, 10), "xy", {"sheet": True}),
+    ((24, 8, 40), (0, 0, 0), "xyz", {"arith": "fma"}),
+    ((64, 88, 16), (9, 0, 0), "yz", {"sheet": True}),
+    ((96, 8, 8), (16, 0, 0), "x", {}),
+])
+def test_brick_equals_split(dims, pml, periodic, kw):
+    want = _grid(dims, "split", 3, pml, periodic, **kw)
+    got = _grid(dims, "auto", 3, pml, periodic, tiling=BRICK, **kw)
+    assert np.abs(want[0]).max() > 0
+    _same(got, want)
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+@pytest.mark.parametrize("dims,pml", [((8, 8, 8), (0, 0, 0)), ((40, 16, 24), (10, 5, 9)),
+                                      ((72, 8, 32), (16, 4, 8))])
+def test_brick_equals_marching_16bit(precision, dims, pml):
+    want = _grid(dims, "fused", 5, pml, precision=precision, tiling=(4, 5, 3))
+    got = _grid(dims, "fused", 5, pml, precision=precision, tiling=BRICK)
+    _same(got, want)
+
+
+def test_default_tiling_round_trips_and_marching_stays_selectable():
+    g = wf.DeviceFieldGrid(wf.GridDims(64, 64, 64))
+    try:
+        assert g.tiling() == BRICK and not g.column_tiles
+        g.set_tiling(*g.tiling())
+        g.step(2)
+        g.set_tiling(4, 12, 3)
+        assert g.tiling() == (4, 12, 3)
+        g.step(2)
+        g.sync()
+    finally:
+        g.close()

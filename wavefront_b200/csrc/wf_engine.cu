@@ -90,7 +90,7 @@ struct wf_handle {
   SrcDev *d_src = nullptr;
   ProbeDev *d_probe = nullptr;
   bool tables_dirty = false;  // d_src / d_probe lag srcs / probes (flush_tables)
-  long long *d_step = nullptr;
+  long long *d_step = nullptr;  // [2]: index of the step that reads state buffer b
   int *d_err = nullptr;
   long long steps_done = 0;
   // learned boundary closure (applied after every step kernel when on)
@@ -112,6 +112,9 @@ struct wf_handle {
   FusedConfig cfg{4, 12, 3};
   int test_extra_tx = 0;      // wf_set_test_stall
   bool cfg_user_set = false;  // otherwise chosen from the grid at first use
+  bool col_user_set = false;  // wf_set_column_tiles was called
+  bool brick = false;         // the step runs as bricks (set with the maps)
+  wf::BrickMaps brick_map[2];  // per state buffer read
   wf::FusedMaps maps[2];      // per state buffer (the one read by the step)
   int *d_items = nullptr;     // work items grouped by kernel class
   int class_off[wf::kFusedClassCount] = {}, class_n[wf::kFusedClassCount] = {};
@@ -335,14 +338,60 @@ bool fused_allowed(const wf_handle *h) {
 bool store16(const wf_handle *h) { return h->precision != WF_PREC_F32; }
 size_t elem_bytes(const wf_handle *h) { return store16(h) ? 2 : 4; }
 
-bool use_fused(const wf_handle *h) {
+// Whether the marching kernels (wf_fused_impl.cuh) can run the handle's step:
+// zero-field boundaries, and CPML profiles of at most 64 slab positions per
+// axis (staged in shared memory).
+bool marching_ok(const wf_handle *h) {
   if (h->kernel_pref == WF_KERNEL_SPLIT) return false;
-  // the fused kernel stages CPML profiles of up to 64 slab positions per axis
-  // in shared memory; thicker layers take the split kernels
   for (const AxisState &A : h->ax)
     if (A.T > 0 && A.W > 64) return false;
   return fused_allowed(h) && encode_fn() != nullptr;
 }
+
+// Whether the brick kernel can: any boundary and slab width with FP32
+// storage; 32-bit cell, id and psi indices, and the grid limits of a launch.
+bool brick_ok(const wf_handle *h) {
+  if (h->kernel_pref == WF_KERNEL_SPLIT || encode_fn() == nullptr) return false;
+  if (store16(h) && !marching_ok(h)) return false;
+  const long long ids = static_cast<long long>(h->mat_pitch) * h->ny * h->nz;
+  return ids < (1ll << 31) && h->nx <= (1 << 19) && h->nz <= (1 << 17);
+}
+
+// The tiling that names the brick step.
+bool is_brick(const FusedConfig &c) {
+  return c.ty == wf::kBrickY && c.zchunk == wf::kBrickZ && c.stages == 1;
+}
+
+// Whether the step runs as bricks rather than as marching tiles (or, where
+// neither can, as the split pair).  Unless the caller chose a tiling or the
+// column tiles, the cheaper of the two by their times on B200, in
+// microseconds per million cells (cubes of 64 to 640 cells, 0- to 16-cell
+// CPML):
+//   FP32, marching  N / 120e3 + 23 us per million CPML cells + 100 us for the
+//                   chain of its slowest class (none without CPML);
+//   FP32, bricks    N / 95e3 + 19 us per million CPML cells
+//                   (256^3, 8-cell CPML: 298 -> 233 us; 64^3: 51.9 -> 6.8;
+//                   512^3, 16-cell: 1747 and 1850, so marching; 512^3 without
+//                   CPML: 1119 and 1364, marching);
+//   16-bit          375 us + 9.2 us per million cells marching against 13.5
+//                   us bricks (320^3: 676 -> 478; 512^3: 1606 and 1812).
+bool use_brick(const wf_handle *h) {
+  if (!brick_ok(h)) return false;
+  if (h->cfg_user_set) return is_brick(h->cfg);
+  if (h->col_user_set) return false;
+  if (!marching_ok(h)) return true;
+  const double n = 1e-6 * static_cast<double>(h->N);
+  if (store16(h)) return n < 86.0;
+  double inner = n;
+  for (int a = 0; a < 3; ++a) {
+    const int len = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz);
+    inner *= static_cast<double>(len - h->ax[a].W) / len;
+  }
+  const double shell = n - inner;
+  return 2.2 * n < (shell > 0.0 ? 100.0 + 4.0 * shell : 4.0);
+}
+
+bool use_fused(const wf_handle *h) { return use_brick(h) || marching_ok(h); }
 
 bool has_pml(const wf_handle *h) { return h->ax[0].T > 0 || h->ax[1].T > 0 || h->ax[2].T > 0; }
 FusedArgs fused_args(const wf_handle *h);
@@ -366,6 +415,34 @@ bool encode(CUtensorMap *m, CUtensorMapDataType t, int rank, void *base, const c
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+}  // namespace
+
+namespace wf {
+
+bool brick_encode(BrickMaps *m, void *fields, int nx, int ny, int nz, int prec) {
+  if (!encode_fn()) return false;
+  unsigned eb[4], hb[4];
+  brick_boxes(prec, eb, hb);
+  const cuuint64_t es = prec == kPrecF32 ? 4 : 2;
+  const cuuint64_t n = static_cast<cuuint64_t>(nx) * ny * nz;
+  const cuuint64_t dim[4] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz, 6};
+  const cuuint64_t str[3] = {nx * es, (cuuint64_t)nx * ny * es, n * es};
+  const CUtensorMapDataType t = prec == kPrecF16    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                : prec == kPrecBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                    : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const cuuint32_t ebox[4] = {eb[0], eb[1], eb[2], eb[3]}, hbox[4] = {hb[0], hb[1], hb[2], hb[3]};
+  return encode(&m->e, t, 4, fields, dim, str, ebox) && encode(&m->h, t, 4, fields, dim, str, hbox);
+}
+
+void brick_geometry(BrickArgs *a) {
+  a->tiles_x = (a->g.nx + kBrickX - 1) / kBrickX;
+  a->x_magic = static_cast<unsigned>(((1ull << 32) + a->tiles_x - 1) / a->tiles_x);  // 2^32 -> 0
+}
+
+}  // namespace wf
+
+namespace {
 
 // Tiling used unless the caller set one: 4 rows, 3 stages, and the z chunk
 // measured best on B200 (two_spheres 512^3, random spheres 1024^3).  A
@@ -401,6 +478,16 @@ wf_status build_maps(wf_handle *h, bool allow_cols = true) {
                                                                 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   const cuuint64_t mdim[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)h->nz};
   const cuuint64_t mstr[2] = {(cuuint64_t)h->mat_pitch, (cuuint64_t)h->mat_pitch * h->ny};
+  h->brick = use_brick(h);
+  if (h->brick) {
+    h->cols = false;
+    for (int b = 0; b < 2; ++b)
+      if (!wf::brick_encode(&h->brick_map[b], h->fld[b], h->nx, h->ny, h->nz, h->precision))
+        return fail(h, WF_ERR_CUDA, "cuTensorMapEncodeTiled(bricks) failed");
+    WF_CUDA(h, wf::brick_prepare(h->precision, h->arith == WF_ARITH_FMA));
+    h->maps_ok = true;
+    return WF_OK;
+  }
   const cuuint32_t ebox[4] = {eb[0], eb[1], eb[2], eb[3]};
   const cuuint32_t hbox[4] = {hb[0], hb[1], hb[2], hb[3]};
   const cuuint32_t mbox[3] = {mb[0], mb[1], mb[2]};
@@ -587,7 +674,8 @@ TailArgs tail_args(const wf_handle *h) {
   t.nsrc = static_cast<int>(h->srcs.size());
   t.probe = h->d_probe;
   t.nprobe = static_cast<int>(h->probes.size());
-  t.step = h->d_step;
+  t.step = h->d_step + h->cur;
+  t.step_next = h->d_step + (h->cur ^ 1);
   t.prec = h->precision;
   t.shift_f = h->shift[h->cur ^ 1];
   t.slab_max = h->slab_max;
@@ -634,8 +722,36 @@ cudaEvent_t timing_event(wf_handle *h) {
   return h->ev_pool[h->ev_used++];
 }
 
+// Whether a brick step applies the sources and probes itself: few of them,
+// and nothing (the closure) between the step and its sources.
+bool brick_tail(const wf_handle *h) {
+  return h->brick && !store16(h) && !h->closure && (!h->srcs.empty() || !h->probes.empty()) &&
+         h->srcs.size() <= wf::kBrickTailMax && h->probes.size() <= wf::kBrickTailMax;
+}
+
+wf::BrickArgs brick_args(const wf_handle *h) {
+  wf::BrickArgs a{};
+  a.g = grid_args(h);
+  wf::brick_geometry(&a);
+  a.test_extra_tx = h->test_extra_tx;
+  if (brick_tail(h)) {
+    a.tail.on = 1;
+    a.tail.nsrc = static_cast<int>(h->srcs.size());
+    a.tail.nprobe = static_cast<int>(h->probes.size());
+    a.tail.src = h->d_src;
+    a.tail.probe = h->d_probe;
+    a.tail.step = h->d_step + h->cur;
+    a.tail.step_next = h->d_step + (h->cur ^ 1);
+  }
+  return a;
+}
+
 wf_status enqueue_one(wf_handle *h) {
   GridArgs g = grid_args(h);
+  if (h->tables_dirty && (!h->srcs.empty() || !h->probes.empty() || store16(h))) {
+    wf_status s = flush_tables(h);
+    if (s != WF_OK) return s;
+  }
   const bool fma = h->arith == WF_ARITH_FMA;
   cudaError_t e;
   if (h->timing) {
@@ -648,10 +764,15 @@ wf_status enqueue_one(wf_handle *h) {
       wf_status s = build_maps(h);
       if (s != WF_OK) return s;
     }
-    if (!h->fork_ev) {
+    if (!h->brick && !h->fork_ev) {
       wf_status s = acquire_streams(h);
       if (s != WF_OK) return s;
     }
+  }
+  if (use_fused(h) && h->brick) {
+    e = wf::launch_brick(h->brick_map[h->cur], brick_args(h), fma, h->stream);
+    if (e == cudaSuccess) h->kernel_launches += 1;
+  } else if (use_fused(h)) {
     const FusedArgs a = fused_args(h);
     // class 0 (interior) on the main stream, the CPML classes on side
     // streams forked from it; they touch disjoint cells of the next state.
@@ -703,11 +824,7 @@ wf_status enqueue_one(wf_handle *h) {
     WF_CUDA(h, cudaEventRecord(ev, h->stream));
   }
   // 16-bit storage always runs the tail: it picks the next step's shifts
-  if (!h->srcs.empty() || !h->probes.empty() || store16(h)) {
-    if (h->tables_dirty) {
-      wf_status s = flush_tables(h);
-      if (s != WF_OK) return s;
-    }
+  if ((!h->srcs.empty() || !h->probes.empty() || store16(h)) && !brick_tail(h)) {
     e = wf::launch_tail(tail_args(h), h->stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "tail kernel launch");
     h->kernel_launches += 1;
@@ -1161,8 +1278,8 @@ wf_status wf_create(const wf_grid_desc *d, wf_handle **out) {
       (e = cudaMemsetAsync(h->mat, 0, mbytes, h->stream)) != cudaSuccess ||
       (e = wf::dev_alloc(&h->coef, sizeof(float4) * 256)) != cudaSuccess ||
       (e = cudaMemsetAsync(h->coef, 0, sizeof(float4) * 256, h->stream)) != cudaSuccess ||
-      (e = wf::dev_alloc(&h->d_step, sizeof(long long))) != cudaSuccess ||
-      (e = cudaMemsetAsync(h->d_step, 0, sizeof(long long), h->stream)) != cudaSuccess ||
+      (e = wf::dev_alloc(&h->d_step, 2 * sizeof(long long))) != cudaSuccess ||
+      (e = cudaMemsetAsync(h->d_step, 0, 2 * sizeof(long long), h->stream)) != cudaSuccess ||
       (e = wf::dev_alloc(&h->d_err, sizeof(int))) != cudaSuccess ||
       (e = cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream)) != cudaSuccess)
     return cleanup_fail(cuda_fail(nullptr, e, "cudaMalloc(state)"));
@@ -1481,7 +1598,7 @@ wf_status wf_step(wf_handle *h, int nsteps) {
     wf_status s = build_maps(h);
     if (s != WF_OK) return s;
   }
-  if (use_fused(h) && !h->fork_ev) {  // the side streams, outside any capture too
+  if (use_fused(h) && !h->brick && !h->fork_ev) {  // the side streams, outside any capture too
     wf_status s = acquire_streams(h);
     if (s != WF_OK) return s;
   }
@@ -1827,7 +1944,9 @@ wf_status wf_set_test_stall(wf_handle *h, int extra_bytes) {
 
 wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out) {
   if (!h || !out) return WF_ERR_ARG;
-  const FusedConfig c = h->cfg_user_set ? h->cfg : default_cfg(h);
+  const FusedConfig c = h->cfg_user_set ? h->cfg
+                        : use_brick(h)  ? FusedConfig{wf::kBrickY, wf::kBrickZ, 1}
+                                        : default_cfg(h);
   out->tile_rows = c.ty;
   out->z_chunk = c.zchunk;
   out->stages = c.stages;
@@ -1837,7 +1956,8 @@ wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out) {
 wf_status wf_set_tiling(wf_handle *h, const wf_tiling *t) {
   if (!h || !t) return fail(h, WF_ERR_ARG, "null argument");
   FusedConfig c{t->tile_rows, t->z_chunk, t->stages};
-  if (!wf::fused_supported(c, h->precision)) return fail(h, WF_ERR_ARG, "tiling not instantiated");
+  if (!wf::fused_supported(c, h->precision) && !(is_brick(c) && brick_ok(h)))
+    return fail(h, WF_ERR_ARG, "tiling not instantiated");
   DeviceGuard guard(h->dev);
   WF_CUDA(h, cudaStreamSynchronize(h->stream));
   drop_graphs(h);
@@ -1854,6 +1974,7 @@ wf_status wf_set_column_tiles(wf_handle *h, int enable) {
   WF_CUDA(h, cudaStreamSynchronize(h->stream));
   drop_graphs(h);
   h->col_pref = enable != 0;
+  h->col_user_set = true;
   ++h->version;
   h->maps_ok = false;
   return WF_OK;
@@ -1861,13 +1982,13 @@ wf_status wf_set_column_tiles(wf_handle *h, int enable) {
 
 int wf_column_tiles_active(const wf_handle *h) {
   if (!h) return -1;
-  if (!use_fused(h)) return 0;
+  if (!use_fused(h) || use_brick(h)) return 0;
   return (h->maps_ok ? h->cols : cols_apply(h)) ? 1 : 0;
 }
 
 wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) {
   if (!h || steps <= 0) return fail(h, WF_ERR_ARG, "bad autotune arguments");
-  if (!use_fused(h)) return fail(h, WF_ERR_UNSUPPORTED, "autotuning applies to the fused kernel");
+  if (!marching_ok(h)) return fail(h, WF_ERR_UNSUPPORTED, "autotuning applies to the fused kernel");
   if (h->steps_done != 0)
     return fail(h, WF_ERR_STATE, "autotune before the first step (it runs trial steps)");
   DeviceGuard guard(h->dev);
@@ -1879,6 +2000,7 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   const int orig_cur = h->cur;
   h->cfg_user_set = true;  // trials and the result are explicit tilings
   std::vector<FusedConfig> cands;
+  if (brick_ok(h)) cands.push_back(FusedConfig{wf::kBrickY, wf::kBrickZ, 1});
   const int tys[] = {4, 8, 16};
   const int stg[] = {3, 4};
   const int zcs[] = {16, 32, 64, 128, 1 << 20};
@@ -1931,7 +2053,7 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
       if (A.psi[k]) WF_CUDA(h, memset_sync(A.psi[k], 0, sizeof(float) * 4 * A.cells, h->stream));
   WF_CUDA(h, memset_sync(h->d_err, 0, sizeof(int), h->stream));
   if (store16(h)) {  // the trial steps ran the 16-bit tail: rewind its counters
-    WF_CUDA(h, memset_sync(h->d_step, 0, sizeof(long long), h->stream));
+    WF_CUDA(h, memset_sync(h->d_step, 0, 2 * sizeof(long long), h->stream));
     WF_CUDA(h, memset_sync(h->d_ovf, 0, sizeof(unsigned long long), h->stream));
   }
   if (best) {
@@ -2466,8 +2588,8 @@ wf_status wf_checkpoint_load(wf_handle *h, const char *path) {
   }
   if (sum.v != c.checksum) return fail(h, WF_ERR_IO, "checkpoint checksum mismatch");
   h->steps_done = c.steps_done;
-  const long long step = c.steps_done;
-  WF_CUDA(h, h2d_sync(h->d_step, &step, sizeof(step), h->stream));
+  const long long step[2] = {c.steps_done, c.steps_done};
+  WF_CUDA(h, h2d_sync(h->d_step, step, sizeof(step), h->stream));
   if (store16(h)) {
     const unsigned long long ovf = c.ovf;
     WF_CUDA(h, h2d_sync(h->d_ovf, &ovf, sizeof(ovf), h->stream));

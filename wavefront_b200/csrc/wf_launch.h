@@ -15,7 +15,8 @@ struct TailArgs {
   int nsrc;
   const ProbeDev *probe;
   int nprobe;
-  long long *step;  // device step counter (read, then incremented)
+  const long long *step;  // index of this step (device)
+  long long *step_next;   // receives the next step's index
   // 16-bit storage: shifts of the new state (sources and probes decode and
   // re-encode with them), its slab maxima, and the shifts the next step
   // writes with (computed here, into the buffer the step just read)
@@ -40,6 +41,44 @@ struct FusedArgs {
   int prof_in_smem;  // every CPML axis has at most 64 slab positions
   int test_extra_tx;  // testing aid: bytes stage 0 expects beyond its copies (0 normally)
 };
+
+// Brick step (wf_brick_impl.cuh): one CTA per brick of cells.
+constexpr int kBrickX = 32, kBrickY = 8, kBrickZ = 4;
+
+// Sources and probes a brick step applies itself (on = 0: none, or a k_tail
+// launch follows): at most 32 of each.  step: the index of this step, read;
+// step_next (another word) receives the next one's.
+struct BrickTail {
+  int on, nsrc, nprobe;
+  const SrcDev *src;
+  const ProbeDev *probe;
+  const long long *step;
+  long long *step_next;
+};
+constexpr int kBrickTailMax = 32;
+
+struct BrickArgs {
+  GridArgs g;
+  int tiles_x;
+  unsigned x_magic;   // ceil(2^32 / tiles_x), i / tiles_x as a high product (0: tiles_x is 1)
+  int test_extra_tx;  // as in FusedArgs
+  BrickTail tail;
+};
+
+struct BrickMaps {
+  CUtensorMap e, h;
+};
+// Encodes the maps over a state of 6*nx*ny*nz values (16-byte aligned), and
+// fills a->tiles_x and x_magic from a->g (wf_engine.cu).
+bool brick_encode(BrickMaps *m, void *fields, int nx, int ny, int nz, int prec);
+void brick_geometry(BrickArgs *a);
+// TMA boxes of a brick's E and H
+void brick_boxes(int prec, unsigned e_box[4], unsigned h_box[4]);
+cudaError_t brick_prepare(int prec, bool fma);
+cudaError_t launch_brick(const BrickMaps &m, const BrickArgs &a, bool fma, cudaStream_t s);
+
+cudaError_t brick16_prepare(int prec);  // wf_brick16.cu
+cudaError_t brick16_launch(const BrickMaps &m, const BrickArgs &a, cudaStream_t s);
 
 // Tiling of the fused kernel: TY rows per CTA (x width kTileX), z chunk and
 // pipeline depth.  Only the instantiated combinations are accepted.

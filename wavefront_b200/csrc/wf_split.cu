@@ -316,7 +316,7 @@ __device__ void tail_body(const TailArgs &t, float *s_src) {
   }
   __syncthreads();
   if (f16) next_shifts(t, st + 1, s_src, true);
-  if (threadIdx.x == 0) *t.step = st + 1;
+  if (threadIdx.x == 0) *t.step_next = st + 1;
 }
 
 __global__ void k_next_shifts(TailArgs t, long long next) {

@@ -3,10 +3,10 @@
   convergence_study()     examples/convergence_study.rs:204-369
   pml_reflection_study()  examples/pml_reflection_study.rs:237-387
 
-Both drive a 1D plane wave in an nx x 8 x 8 vacuum domain with periodic Y/Z
-(the split kernels handle periodic axes), a hard Ez sheet source and a probe
-trace, then post-process in the reference's f32/f64 arithmetic (libm for
-sinf/asinf/log10f, as the reference's f32 methods call).
+Both drive a 1D plane wave in an nx x 8 x 8 vacuum domain with periodic Y/Z,
+a hard Ez sheet source and a probe trace, then post-process in the reference's
+f32/f64 arithmetic (libm for sinf/asinf/log10f, as the reference's f32 methods
+call).
 """
 from __future__ import annotations
 
@@ -44,7 +44,7 @@ def plane_wave_trace(nx: int, dx, dt, freq, x_source: int, x_probe: int, steps: 
                      pml_voxels: int, device: int = 0) -> np.ndarray:
     """run_plane_wave of both studies on the GPU; returns the f32 Ez trace."""
     dims = GridDims(nx, 8, 8)
-    g = DeviceFieldGrid(dims, boundary=("zero", "periodic", "periodic"), kernel="split",
+    g = DeviceFieldGrid(dims, boundary=("zero", "periodic", "periodic"),
                         device=device)
     try:
         g.set_materials(MaterialGrid(dims), MaterialTable.vacuum_filled(float(dt), float(dx)))
