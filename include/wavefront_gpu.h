@@ -403,7 +403,7 @@ int64_t wf_nn_tensor_core_timeouts(void);
 /* ---- batched stepping (no reference counterpart) ------------------------ */
 
 /* Many independent grids of uneven size stepped together: each step is one
- * persistent kernel launch over the work items (tile x z chunk) of every
+ * kernel launch over the work items (bricks, or tile x z chunk) of every
  * grid, then one tail launch for every grid's sources and probes; runs of
  * 32 steps replay a captured CUDA graph.  The grids are ordinary handles,
  * created on the batch's stream: set them up and read them back with the
@@ -427,7 +427,10 @@ wf_status wf_batch_get_tiling(const wf_batch *b, wf_tiling *out);
 wf_status wf_batch_set_tiling(wf_batch *b, const wf_tiling *t);
 /* Times the batched step kernel for `steps` steps under each instantiated
  * tiling and z chunk, keeps the fastest, and restores every grid's fields
- * and psi (sources and probes do not run during the trials). */
+ * and psi (sources and probes do not run during the trials).  The brick step,
+ * a new batch's default, is timed too and stays in use (wf_batch_get_tiling
+ * {8, 4, 1}) when no z-march beats it; best and best_ms always describe the
+ * fastest z-march. */
 wf_status wf_batch_autotune(wf_batch *b, int steps, wf_tiling *best, float *best_ms);
 
 /* ---- device memory cache (no reference counterpart) ---------------------- */

@@ -278,3 +278,37 @@ def test_ablation_closure_on_the_thin_layer(trained):
           f"plain 4-cell CPML {steep4['max_rel_error']:.3f}, 16-cell CPML {thick16['max_rel_error']:.4f}")
     assert np.isfinite(closed["max_rel_error"])
     assert closed["max_rel_error"] < 0.5 * thin["max_rel_error"]
+
+
+@pytest.mark.parametrize("n,ci,co,d,h,w,nface", [
+    (1, 1, 1, 1, 1, 1, 1), (3, 16, 16, 8, 16, 16, 2), (5, 10, 16, 5, 7, 19, 6),
+    (40, 16, 6, 8, 5, 33, 6), (2, 3, 5, 9, 4, 17, 8), (70, 2, 3, 2, 3, 4, 3)])
+def test_weight_gradient_against_float64(n, ci, co, d, h, w, nface):
+    """dw adds to what is there; samples whose face is not below nface are left
+    out.  Tolerance: FP32 sums of at most n*d*h*w products, error below
+    2 * sqrt(terms) * 2^-24 of the sum of magnitudes, plus the final add."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    from wavefront_b200 import lib
+    g = torch.Generator(device="cuda").manual_seed(n * 1000 + w)
+    x = torch.randn(n, ci, d, h, w, device="cuda", generator=g)
+    dz = torch.randn(n, co, d, h, w, device="cuda", generator=g)
+    face = torch.randint(0, nface + 1, (n,), device="cuda", generator=g).to(torch.int32)
+    dw = torch.randn(nface, co, ci, 27, device="cuda", generator=g)
+    want, mag = dw.double().clone(), dw.double().abs()
+    xp = torch.nn.functional.pad(x.double(), (1, 1, 1, 1, 1, 1))
+    for s in range(n):
+        f = int(face[s])
+        if f >= nface:
+            continue
+        for t in range(27):
+            a, b, c = t // 9, t // 3 % 3, t % 3
+            win = xp[s, :, a:a + d, b:b + h, c:c + w]
+            want[f, :, :, t] += torch.einsum("odhw,cdhw->oc", dz[s].double(), win)
+            mag[f, :, :, t] += torch.einsum("odhw,cdhw->oc", dz[s].double().abs(), win.abs())
+    p = lambda t: C.c_void_p(t.data_ptr())
+    st = lib().wf_nn_conv3d_backward_weight(p(x), p(dz), p(face), p(dw), n, ci, co, d, h, w, nface,
+                                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    tol = 2.0 * (n * d * h * w + 1) ** 0.5 * 2.0 ** -24
+    assert ((dw.double() - want).abs() <= tol * mag + 1e-30).all()

@@ -20,4 +20,22 @@ cudaError_t launch_brick(const BrickMaps &m, const BrickArgs &a, bool fma, cudaS
   return fma ? brick_launch_t<true, float>(m, a, s) : brick_launch_t<false, float>(m, a, s);
 }
 
+cudaError_t brick_batch_prepare() {
+  cudaError_t e = cudaFuncSetAttribute(k_brick_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       BrickL<float>::BYTES);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_brick_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              BrickL<float>::BYTES);
+}
+
+cudaError_t launch_brick_batch(const BrickScene *scenes, const int4 *items, int n_items, int parity,
+                               bool xs, cudaStream_t s) {
+  if (n_items <= 0) return cudaSuccess;
+  if (xs)
+    k_brick_batch<true><<<n_items, kBrickThreads, BrickL<float>::BYTES, s>>>(scenes, items, parity);
+  else
+    k_brick_batch<false><<<n_items, kBrickThreads, BrickL<float>::BYTES, s>>>(scenes, items, parity);
+  return cudaGetLastError();
+}
+
 }  // namespace wf

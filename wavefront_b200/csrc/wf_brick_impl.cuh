@@ -720,6 +720,26 @@ __global__ void __launch_bounds__(kBrickThreads, PML ? 2 : 3)
   brick_body<FMA, PML, XS, ST>(&tmE, &tmH, a, smem, x0, y0, blockIdx.y * kBrickZ);
 }
 
+// Batched step: CTA i computes brick items[i] = (scene, x0, y0, z0).  The
+// scene's arguments are copied to shared memory first: constant-bank operands
+// of k_brick become shared loads here.
+template <bool XS>
+__global__ void __launch_bounds__(kBrickThreads, 2)
+    k_brick_batch(const BrickScene *scenes, const int4 *items, int parity) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
+  __shared__ BrickArgs s_args;
+  const int4 it = __ldg(items + blockIdx.x);
+  const BrickScene *sc = scenes + it.x;
+  const int *src = reinterpret_cast<const int *>(&sc->args[parity]);
+  for (int i = threadIdx.x; i < static_cast<int>(sizeof(BrickArgs) / 4); i += kBrickThreads)
+    reinterpret_cast<int *>(&s_args)[i] = __ldg(src + i);
+  __syncthreads();
+  brick_body<false, true, XS, float>(&sc->maps[parity].e, &sc->maps[parity].h, s_args, smem, it.y, it.z,
+                                     it.w);
+}
+
 template <bool FMA, typename ST>
 cudaError_t brick_prepare_t() {
   const void *fns[] = {(const void *)k_brick<FMA, false, false, ST>,

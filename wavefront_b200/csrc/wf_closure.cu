@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "wf_band.cuh"
 #include "wf_closure.h"
 
@@ -192,42 +194,106 @@ __global__ void k_conv_bwd_data(const float *dz, const __nv_bfloat16 *w, const i
 }
 
 // dw[face][co][ci][tap] += sum over samples of that face and voxels p of
-// dz[n][co][p] * in[n][ci][p + tap]: one thread per weight entry, the
-// samples split over blockIdx.y (partial sums added atomically)
-__global__ void k_conv_bwd_weight(const float *in, const float *dz, const int *face, float *dw,
-                                  int n, int ci, int co, int D, int H, int W, int nface) {
-  const int nw = co * ci * kTaps;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nw) return;
-  const int o = e / (ci * kTaps), c = (e / kTaps) % ci, t = e % kTaps;
-  const int od = t / 9 - 1, oy = (t / 3) % 3 - 1, ox = t % 3 - 1;
+// dz[n][co][p] * in[n][ci][p + tap].
+//
+// A CTA works for one face (blockIdx.y) on every gridDim.x-th tile of the
+// face's samples: 4 planes x 4 rows x 16 columns of dz and their haloed input
+// in shared memory.  A thread owns one input channel, two output channels and
+// all 27 taps (54 sums kept in registers over all its tiles): a row of 4
+// columns takes one 128-bit load per output channel and two per tap row for
+// 216 FMAs, so the FMA pipes bound it.  Threads beyond ci * co / 2 split the
+// tile's rows between them; the sums meet in global memory once per CTA.
+// Measured on B200 (a training step on 128 samples of 8 x 16 x 16): 4.37 ms, of
+// which the three layers' weight gradients took 0.69 + 1.59 + 1.44 ms with one
+// thread per weight reading both operands from global memory; 1.23 ms now.
+constexpr int kBwD = 4, kBwY = 4, kBwX = 16;         // tile of dz
+constexpr int kBwRow = 20;                           // input row: 18 columns, 16-byte pitch
+constexpr int kBwIn = (kBwD + 2) * (kBwY + 2) * kBwRow + 4;  // one input channel; + 4: channels
+constexpr int kBwDz = kBwD * kBwY * kBwX + 4;                // start in different banks
+constexpr int kBwSmem = 16 * (kBwIn + kBwDz) * 4;
+constexpr int kBwThreads = 256;
+
+__global__ void __launch_bounds__(kBwThreads, 2)
+    k_conv_bwd_weight(const float *in, const float *dz, const int *face, float *dw, int n, int ci,
+                      int co, int D, int H, int W) {
+  extern __shared__ __align__(16) float s_t[];
+  float *s_in = s_t, *s_dz = s_t + 16 * kBwIn;
+  const int f = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int co2 = (co + 1) / 2, combos = ci * co2, parts = kBwThreads / combos;
+  const int combo = tid % combos, part = tid / combos;
+  const int c = combo % ci, o = 2 * (combo / ci);
+  const bool active = part < parts;
+  const int tx = (W + kBwX - 1) / kBwX, ty = (H + kBwY - 1) / kBwY, td = (D + kBwD - 1) / kBwD;
+  const int tiles = tx * ty * td;
   const long long P = static_cast<long long>(D) * H * W;
-  float acc[8];
-  for (int f = 0; f < 8; ++f) acc[f] = 0.0f;
-  for (int s = blockIdx.y; s < n; s += gridDim.y) {
-    const int f = face ? face[s] : 0;
-    const float *g = dz + (static_cast<long long>(s) * co + o) * P;
-    const float *v = in + (static_cast<long long>(s) * ci + c) * P;
-    float sum = 0.0f;
-    for (int d = 0; d < D; ++d) {
-      const int dd = d + od;
-      if (dd < 0 || dd >= D) continue;
-      for (int y = 0; y < H; ++y) {
-        const int yy = y + oy;
-        if (yy < 0 || yy >= H) continue;
-        const float *gr = g + (static_cast<long long>(d) * H + y) * W;
-        const float *vr = v + (static_cast<long long>(dd) * H + yy) * W;
-        for (int x = 0; x < W; ++x) {
-          const int xx = x + ox;
-          if (xx < 0 || xx >= W) continue;
-          sum = __fmaf_rn(gr[x], vr[xx], sum);
+  float acc0[27], acc1[27];
+#pragma unroll
+  for (int t = 0; t < 27; ++t) acc0[t] = acc1[t] = 0.0f;
+  bool any = false;
+  long long count = 0;  // tiles of this face so far
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const int mine = s0 + lane < n ? (face ? face[s0 + lane] : 0) : -1;
+    for (unsigned m = __ballot_sync(0xffffffffu, mine == f); m; m &= m - 1, count += tiles) {
+      const int s = s0 + __ffs(m) - 1;
+      // this CTA's tiles of the sample: those with (count + q) % gridDim.x == blockIdx.x
+      int q = static_cast<int>((blockIdx.x + gridDim.x - count % gridDim.x) % gridDim.x);
+      for (; q < tiles; q += gridDim.x) {
+        const int x0 = q % tx * kBwX, y0 = q / tx % ty * kBwY, d0 = q / (tx * ty) * kBwD;
+        any = true;
+        __syncthreads();  // the tile before is consumed
+        const float *src = in + static_cast<long long>(s) * ci * P;
+        for (int i = tid; i < ci * (kBwD + 2) * (kBwY + 2) * kBwRow; i += kBwThreads) {
+          const int k = i % kBwRow, row = i / kBwRow % ((kBwD + 2) * (kBwY + 2)),
+                    ch = i / (kBwRow * (kBwD + 2) * (kBwY + 2));
+          const int d = d0 - 1 + row / (kBwY + 2), y = y0 - 1 + row % (kBwY + 2), x = x0 - 1 + k;
+          const bool ok = d >= 0 && d < D && y >= 0 && y < H && x >= 0 && x < W && k < kBwX + 2;
+          s_in[ch * kBwIn + row * kBwRow + k] =
+              ok ? __ldg(src + ch * P + (static_cast<long long>(d) * H + y) * W + x) : 0.0f;
+        }
+        const float *g = dz + static_cast<long long>(s) * co * P;
+        for (int i = tid; i < 2 * co2 * kBwD * kBwY * kBwX; i += kBwThreads) {
+          const int k = i % kBwX, row = i / kBwX % (kBwD * kBwY), ch = i / (kBwX * kBwD * kBwY);
+          const int d = d0 + row / kBwY, y = y0 + row % kBwY, x = x0 + k;
+          const bool ok = ch < co && d < D && y < H && x < W;
+          s_dz[ch * kBwDz + row * kBwX + k] =
+              ok ? __ldg(g + ch * P + (static_cast<long long>(d) * H + y) * W + x) : 0.0f;
+        }
+        __syncthreads();
+        if (!active) continue;
+        for (int row = part; row < kBwD * kBwY; row += parts) {
+          const float *z0 = s_dz + o * kBwDz + row * kBwX;
+          const float *v = s_in + c * kBwIn + (row / kBwY * (kBwY + 2) + row % kBwY) * kBwRow;
+#pragma unroll 1
+          for (int x = 0; x < kBwX; x += 4) {
+            const float4 ga = *reinterpret_cast<const float4 *>(z0 + x);
+            const float4 gb = *reinterpret_cast<const float4 *>(z0 + kBwDz + x);
+            const float g0[4] = {ga.x, ga.y, ga.z, ga.w}, g1[4] = {gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+            for (int r = 0; r < 9; ++r) {  // tap rows (dz, dy)
+              const float *w = v + (r / 3 * (kBwY + 2) + r % 3) * kBwRow + x;
+              const float4 a = *reinterpret_cast<const float4 *>(w);
+              const float2 b = *reinterpret_cast<const float2 *>(w + 4);
+              const float e[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+#pragma unroll
+              for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  acc0[3 * r + k] = __fmaf_rn(g0[i], e[i + k], acc0[3 * r + k]);
+                  acc1[3 * r + k] = __fmaf_rn(g1[i], e[i + k], acc1[3 * r + k]);
+                }
+            }
+          }
         }
       }
     }
-    if (f < 8) acc[f] += sum;
   }
-  for (int f = 0; f < nface && f < 8; ++f)
-    if (acc[f] != 0.0f) atomicAdd(dw + static_cast<long long>(f) * nw + e, acc[f]);
+  if (!any || !active) return;
+  float *out = dw + ((static_cast<long long>(f) * co + o) * ci + c) * kTaps;
+#pragma unroll
+  for (int t = 0; t < 27; ++t) {
+    atomicAdd(out + t, acc0[t]);
+    if (o + 1 < co) atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+  }
 }
 
 __global__ void k_gelu_bwd(const float *da, const float *z, float *dz, long long m) {
@@ -483,10 +549,21 @@ int nn_conv_bwd_data(const float *dz, const void *w_bf16, const int *face, float
 int nn_conv_bwd_weight(const float *in, const float *dz, const int *face, float *dw, int n, int ci,
                        int co, int D, int H, int W, int nface, void *stream) {
   if (ci > kMaxC || co > kMaxC || nface > 8 || n < 1) return cudaErrorInvalidValue;
-  const int nw = co * ci * kTaps;
-  dim3 grid(blocks_for(nw, 128), n < 64 ? n : 64);
-  k_conv_bwd_weight<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(in, dz, face, dw, n, ci, co,
-                                                                         D, H, W, nface);
+  if (ci < 1 || co < 1 || nface < 1 || D < 1 || H < 1 || W < 1) return cudaSuccess;  // nothing to add
+  cudaError_t e = cudaFuncSetAttribute(k_conv_bwd_weight, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kBwSmem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, nsm = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  // two CTAs per SM over the faces, never more than there are tiles
+  const long long tiles = static_cast<long long>(n) * ((W + kBwX - 1) / kBwX) *
+                          ((H + kBwY - 1) / kBwY) * ((D + kBwD - 1) / kBwD);
+  const long long want = std::max(1, 2 * nsm / nface);
+  dim3 grid(static_cast<unsigned>(std::min(want, tiles)), nface);
+  k_conv_bwd_weight<<<grid, kBwThreads, kBwSmem, static_cast<cudaStream_t>(stream)>>>(in, dz, face, dw, n,
+                                                                                      ci, co, D, H, W);
   return cudaGetLastError();
 }
 

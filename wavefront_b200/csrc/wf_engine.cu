@@ -935,8 +935,12 @@ struct wf_batch {
   int dev = 0;
   cudaStream_t stream = nullptr;
   std::vector<wf_handle *> h;
-  FusedConfig cfg{4, 16, 3};
+  FusedConfig cfg{wf::kBrickY, wf::kBrickZ, 1};  // bricks unless a tiling is set
   wf::BatchScene *d_scenes = nullptr;
+  // brick form: the grids' maps and arguments, one item per brick
+  wf::BrickScene *d_bricks = nullptr;
+  int4 *d_brick_items = nullptr;
+  bool brick = false, brick_xs = false;
   int2 *d_items = nullptr;  // grouped by CPML class
   int n_items = 0;
   int class_off[wf::kFusedClassCount] = {}, class_n[wf::kFusedClassCount] = {};
@@ -966,8 +970,12 @@ void batch_drop(wf_batch *b) {
   }
   wf::dev_free(b->d_scenes);
   wf::dev_free(b->d_items);
+  wf::dev_free(b->d_bricks);
+  wf::dev_free(b->d_brick_items);
   wf::dev_free(b->d_tails[0]);
   wf::dev_free(b->d_tails[1]);
+  b->d_bricks = nullptr;
+  b->d_brick_items = nullptr;
   b->d_scenes = nullptr;
   b->d_items = nullptr;
   b->d_tails[0] = b->d_tails[1] = nullptr;
@@ -1042,13 +1050,22 @@ wf_status batch_build(wf_batch *b) {
   std::vector<TailArgs> tails[2];
   b->have_tail = false;
   b->narrow = wf::fused_batch_narrow(b->cfg);
+  b->brick = is_brick(b->cfg);
+  b->brick_xs = false;
+  std::vector<wf::BrickScene> bricks(b->brick ? n : 0);
   for (size_t i = 0; i < n; ++i) {
     wf_handle *h = b->h[i];
     for (const AxisState &A : h->ax)
       if (A.T > 0 && A.W > 64)
         return fail(nullptr, WF_ERR_UNSUPPORTED, "batched grids need CPML slabs of at most 64 cells");
-    wf_status st;
-    if (b->narrow) {
+    wf_status st = WF_OK;
+    if (b->brick) {
+      if (!brick_ok(h)) return fail(nullptr, WF_ERR_UNSUPPORTED, "a batched grid is too large for bricks");
+      for (int p = 0; p < 2; ++p)
+        if (!wf::brick_encode(&bricks[i].maps[p], h->fld[p], h->nx, h->ny, h->nz, h->precision))
+          return fail(nullptr, WF_ERR_CUDA, "cuTensorMapEncodeTiled(brick batch) failed");
+      if (h->ax[0].T % 4) b->brick_xs = true;
+    } else if (b->narrow) {
       st = narrow_batch_maps(h, b->cfg.zchunk, &scenes[i]);
     } else {
       h->cfg = b->cfg;
@@ -1060,7 +1077,13 @@ wf_status batch_build(wf_batch *b) {
     const int cur = h->cur;
     for (int p = 0; p < 2; ++p) {
       h->cur = p;
-      if (!b->narrow) {
+      if (b->brick) {
+        wf::BrickArgs &a = bricks[i].args[p];
+        a = wf::BrickArgs{};
+        a.g = grid_args(h);
+        wf::brick_geometry(&a);
+        a.test_extra_tx = h->test_extra_tx;
+      } else if (!b->narrow) {
         scenes[i].args[p] = fused_args(h);
         scenes[i].maps[p][0] = h->maps[p].e;
         scenes[i].maps[p][1] = h->maps[p].h;
@@ -1070,6 +1093,7 @@ wf_status batch_build(wf_batch *b) {
     }
     h->cur = cur;
     if (!h->srcs.empty() || !h->probes.empty()) b->have_tail = true;
+    if (b->brick) continue;
     const FusedArgs &a = scenes[i].args[0];
     const int nit = a.tiles_x * a.tiles_y * ((h->nz + a.zchunk - 1) / a.zchunk);
     for (int k = 0; k < nit; ++k)
@@ -1078,6 +1102,37 @@ wf_status batch_build(wf_batch *b) {
   }
   std::vector<int2> items;
   b->step_kernels = 0;
+  if (b->brick) {
+    // grid by grid, largest first, each in the single-grid order (x, 8 rows of
+    // bricks in y, z, the next rows): neighbours run close together in time
+    std::vector<int4> list;
+    std::vector<int> gorder(n);
+    for (size_t i = 0; i < n; ++i) gorder[i] = static_cast<int>(i);
+    std::stable_sort(gorder.begin(), gorder.end(), [b](int p, int q) { return b->h[p]->N > b->h[q]->N; });
+    for (int i : gorder) {
+      const wf_handle *h = b->h[i];
+      const int band = 8 * wf::kBrickY;
+      for (int yb = 0; yb < h->ny; yb += band)
+        for (int z = 0; z < h->nz; z += wf::kBrickZ)
+          for (int y = yb; y < std::min(yb + band, h->ny); y += wf::kBrickY)
+            for (int x = 0; x < h->nx; x += wf::kBrickX) list.push_back(make_int4(i, x, y, z));
+    }
+    b->step_kernels = 1;
+    b->n_items = static_cast<int>(list.size());
+    WF_CUDA(nullptr, wf::dev_alloc(&b->d_bricks, sizeof(wf::BrickScene) * n));
+    WF_CUDA(nullptr, h2d_sync(b->d_bricks, bricks.data(), sizeof(wf::BrickScene) * n, b->stream));
+    WF_CUDA(nullptr, wf::dev_alloc(&b->d_brick_items, sizeof(int4) * list.size()));
+    WF_CUDA(nullptr, h2d_sync(b->d_brick_items, list.data(), sizeof(int4) * list.size(), b->stream));
+    WF_CUDA(nullptr, wf::brick_batch_prepare());
+    for (int p = 0; p < 2; ++p) {
+      WF_CUDA(nullptr, wf::dev_alloc(&b->d_tails[p], sizeof(TailArgs) * n));
+      WF_CUDA(nullptr, h2d_sync(b->d_tails[p], tails[p].data(), sizeof(TailArgs) * n, b->stream));
+    }
+    b->versions.clear();
+    for (wf_handle *h : b->h) b->versions.push_back(h->version);
+    b->built = true;
+    return WF_OK;
+  }
   if (b->narrow) {
     // one list, grid by grid (largest grids first), and within a grid its
     // costliest items first (three CPML axes ... interior), each class in
@@ -1132,6 +1187,11 @@ wf_status batch_build(wf_batch *b) {
 // per non-empty class, class 0 on the batch's stream and the others on side
 // streams forked from it and joined back; the classes write disjoint cells.
 wf_status batch_kernel(wf_batch *b, int cur) {
+  if (b->brick) {
+    WF_CUDA(nullptr, wf::launch_brick_batch(b->d_bricks, b->d_brick_items, b->n_items, cur, b->brick_xs,
+                                            b->stream));
+    return WF_OK;
+  }
   WF_CUDA(nullptr, cudaMemsetAsync(b->d_counter, 0, sizeof(int) * wf::kFusedClassCount, b->stream));
   if (b->narrow) {
     WF_CUDA(nullptr, wf::launch_fused_batch_narrow(b->d_scenes, b->d_items, b->n_items, b->d_counter,
@@ -2678,7 +2738,7 @@ wf_handle *wf_batch_handle(wf_batch *b, int i) {
 wf_status wf_batch_set_tiling(wf_batch *b, const wf_tiling *t) {
   if (!b || !t) return fail(nullptr, WF_ERR_ARG, "null argument");
   FusedConfig c{t->tile_rows, t->z_chunk, t->stages};
-  if (!wf::fused_supported(c, wf::kPrecF32) && !wf::fused_batch_narrow(c))
+  if (!wf::fused_supported(c, wf::kPrecF32) && !wf::fused_batch_narrow(c) && !is_brick(c))
     return fail(nullptr, WF_ERR_ARG, "tiling not instantiated");
   DeviceGuard guard(b->dev);
   WF_CUDA(nullptr, cudaStreamSynchronize(b->stream));
@@ -2799,34 +2859,39 @@ wf_status wf_batch_autotune(wf_batch *b, int steps, wf_tiling *best, float *best
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
+  auto trial = [&](const FusedConfig &c) {  // milliseconds a step, or < 0
+    batch_drop(b);
+    b->cfg = c;
+    if (batch_build(b) != WF_OK) return -1.0f;
+    int parity = cur0;
+    bool okc = batch_kernel(b, parity) == WF_OK;  // warm-up
+    parity ^= 1;
+    cudaEventRecord(e0, b->stream);
+    for (int i = 0; i < steps && okc; ++i, parity ^= 1) okc = batch_kernel(b, parity) == WF_OK;
+    cudaEventRecord(e1, b->stream);
+    if (cudaEventSynchronize(e1) != cudaSuccess || !okc) return -1.0f;
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    return ms / steps;
+  };
   const int tys[] = {4, 8, 16, wf::kColTileRows}, stg[] = {3, 4}, zcs[] = {8, 12, 16, 24, 32, 64, 128};
   for (int ty : tys)
     for (int sg : stg)
       for (int zc : zcs) {
         FusedConfig c{ty, zc, sg};
         if (!wf::fused_supported(c, wf::kPrecF32) && !wf::fused_batch_narrow(c)) continue;
-        batch_drop(b);
-        b->cfg = c;
-        if (batch_build(b) != WF_OK) continue;
-        int parity = cur0;
-        bool okc = batch_kernel(b, parity) == WF_OK;  // warm-up
-        parity ^= 1;
-        cudaEventRecord(e0, b->stream);
-        for (int i = 0; i < steps && okc; ++i, parity ^= 1) okc = batch_kernel(b, parity) == WF_OK;
-        cudaEventRecord(e1, b->stream);
-        if (cudaEventSynchronize(e1) != cudaSuccess || !okc) continue;
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        ms /= steps;
-        if (ms < bms) {
+        const float ms = trial(c);
+        if (ms >= 0.0f && ms < bms) {
           bms = ms;
           bc = c;
         }
       }
+  const FusedConfig bricks{wf::kBrickY, wf::kBrickZ, 1};
+  const float brick_ms = trial(bricks);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   batch_drop(b);
-  b->cfg = bc;
+  b->cfg = brick_ms >= 0.0f && brick_ms <= bms ? bricks : bc;
   size_t k = 0;
   for (wf_handle *h : b->h) {
     cudaMemcpyAsync(h->fld[h->cur], saved[k++], sizeof(float) * 6 * h->N, cudaMemcpyDeviceToDevice,

@@ -77,6 +77,16 @@ void brick_boxes(int prec, unsigned e_box[4], unsigned h_box[4]);
 cudaError_t brick_prepare(int prec, bool fma);
 cudaError_t launch_brick(const BrickMaps &m, const BrickArgs &a, bool fma, cudaStream_t s);
 
+// One grid of a batched brick step, in device memory, per parity of the state
+// read; items: (scene, x0, y0, z0) of every brick.  xs: some grid's x CPML
+// depth is not a multiple of 4.
+struct BrickScene {
+  BrickMaps maps[2];
+  BrickArgs args[2];
+};
+cudaError_t brick_batch_prepare();
+cudaError_t launch_brick_batch(const BrickScene *scenes, const int4 *items, int n_items, int parity,
+                               bool xs, cudaStream_t s);
 cudaError_t brick16_prepare(int prec);  // wf_brick16.cu
 cudaError_t brick16_launch(const BrickMaps &m, const BrickArgs &a, cudaStream_t s);
 
