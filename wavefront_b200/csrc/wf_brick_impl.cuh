@@ -92,13 +92,14 @@ struct PlaneUnits {
 // slab positions, and for x whether the group moves as one vector.
 struct GroupPml {
   int fl;
-  bool xvec;
-  int sx, sy, sz;  // sx: position of the first cell (vector), else unused
+  unsigned xin;    // XS: bit k: cell k is in the x slab
+  bool xvec;       // its x psi move as one vector
+  int sx, sy, sz;  // sx: position cell 0 has, or would have, in the x slab
 };
 
 template <bool XS>
 __device__ __forceinline__ GroupPml group_pml(const GridArgs &g, int fl, int x, int y, int z, bool ok) {
-  GroupPml m{0, false, 0, 0, 0};
+  GroupPml m{0, 0u, false, 0, 0, 0};
   if (!ok) return m;
   if (fl & 1) {
     const PmlAxis &P = g.pml[0];
@@ -108,10 +109,14 @@ __device__ __forceinline__ GroupPml group_pml(const GridArgs &g, int fl, int x, 
       if (s0 >= 0) m.fl |= 1;
       m.xvec = true;
     } else {
-      const int s3 = slab_pos(x + 3, g.nx, P.T, P.W);
-      const int s1 = slab_pos(x + 1, g.nx, P.T, P.W), s2 = slab_pos(x + 2, g.nx, P.T, P.W);
-      if (s0 >= 0 || s1 >= 0 || s2 >= 0 || s3 >= 0) m.fl |= 1;
-      m.xvec = s0 >= 0 && s1 >= 0 && s2 >= 0 && s3 == s0 + 3 && (s0 & 3) == 0;
+      // (nx % 8 == 0: a group meets the low slab or the high one, never both
+      // with a gap between, so its positions are consecutive)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (slab_pos(x + k, g.nx, P.T, P.W) >= 0) m.xin |= 1u << k;
+      if (m.xin) m.fl |= 1;
+      m.sx = x < P.T ? x : x - (g.nx - P.W);
+      m.xvec = m.xin == 15u && (m.sx & 3) == 0;
     }
   }
   if (fl & 2) {
@@ -142,16 +147,14 @@ __device__ __forceinline__ void psi_load(const GridArgs &g, const GroupPml &m, i
   if (!(m.fl & (1 << axis))) return;
   const PmlAxis &P = g.pml[axis];
   const float *c = P.psi_cur + slot * P.cells;
-  const unsigned i = psi_at(g, m, axis, x, y, z) + (axis == 0 && m.xvec ? m.sx : 0);
+  const unsigned i = psi_at(g, m, axis, x, y, z) + (axis == 0 ? m.sx : 0);
   if (!XS || axis != 0 || m.xvec) {
     if (!idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) return;
     unpack(b_ldg4(c + i), q);
   } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int s = slab_pos(x + k, g.nx, P.T, P.W);
-      q[k] = s >= 0 && idx_ok(g.err, static_cast<long long>(i) + s, P.cells) ? __ldg(c + i + s) : 0.0f;
-    }
+    for (int k = 0; k < 4; ++k)
+      q[k] = (m.xin >> k & 1u) && idx_ok(g.err, i + k, P.cells) ? __ldg(c + i + k) : 0.0f;
   }
 }
 
@@ -167,7 +170,7 @@ __device__ __forceinline__ void psi_corr(const GridArgs &g, const GroupPml &m, i
     v = U ? __fmul_rn(pml_corr<FMA>(__fmul_rn(v, u.su), b, a, ik, ps), u.iu)
           : pml_corr<FMA>(v, b, a, ik, ps);
   };
-  const unsigned i = psi_at(g, m, axis, x, y, z) + (axis == 0 && m.xvec ? m.sx : 0);
+  const unsigned i = psi_at(g, m, axis, x, y, z) + (axis == 0 ? m.sx : 0);
   float *o = P.psi_nxt + slot * P.cells;
   if (axis != 0) {
     const int s = axis == 1 ? m.sy : m.sz;
@@ -175,23 +178,25 @@ __device__ __forceinline__ void psi_corr(const GridArgs &g, const GroupPml &m, i
 #pragma unroll
     for (int k = 0; k < 4; ++k) one(d[k], p[k], b, a, ik);
     if (store && idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) b_st4(o + i, p);
-  } else if (!XS) {
-    float b[4], a[4], ik[4];
-    unpack(b_ldg4(P.prof + m.sx), b);
-    unpack(b_ldg4(P.prof + P.W + m.sx), a);
-    unpack(b_ldg4(P.prof + 2 * P.W + m.sx), ik);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) one(d[k], p[k], b[k], a[k], ik[k]);
-    if (store && idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) b_st4(o + i, p);
   } else {
+    float b[4], a[4], ik[4];  // by x coordinate: aligned for every group
+    unpack(b_ldg4(P.full + x), b);
+    unpack(b_ldg4(P.full + g.nx + x), a);
+    unpack(b_ldg4(P.full + 2 * g.nx + x), ik);
+    if (!XS || m.xvec) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int s = m.xvec ? m.sx + k : slab_pos(x + k, g.nx, P.T, P.W);
-      if (s < 0) continue;
-      one(d[k], p[k], __ldg(P.prof + s), __ldg(P.prof + P.W + s), __ldg(P.prof + 2 * P.W + s));
-      if (store && !m.xvec && idx_ok(g.err, static_cast<long long>(i) + s, P.cells)) o[i + s] = p[k];
+      for (int k = 0; k < 4; ++k) one(d[k], p[k], b[k], a[k], ik[k]);
+      if (store && idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) b_st4(o + i, p);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float v = d[k];
+        one(v, p[k], b[k], a[k], ik[k]);
+        const bool in = m.xin >> k & 1u;
+        d[k] = in ? v : d[k];
+        if (store && in && idx_ok(g.err, i + k, P.cells)) o[i + k] = p[k];
+      }
     }
-    if (store && m.xvec && idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) b_st4(o + i, p);
   }
 }
 
@@ -456,7 +461,7 @@ __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtenso
       id = __ldg(reinterpret_cast<const uchar4 *>(m));
   }
   // the H terms' psi: in flight while the boxes arrive
-  GroupPml gm{0, false, 0, 0, 0};
+  GroupPml gm{0, 0u, false, 0, 0, 0};
   Psi6 ps;
   if (PML && role < 3) {
     gm = group_pml<XS>(g, fl, x, y, z, in);

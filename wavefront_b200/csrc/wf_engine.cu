@@ -53,7 +53,8 @@ struct ProbeRec {
 
 struct AxisState {
   int T = 0, W = 0, pitch = 0;
-  float *prof = nullptr;       // [3][W]
+  float *prof = nullptr;       // [3][W], then on the x axis [3][nx]
+  const float *full = nullptr;  // that second part
   float *psi[2] = {nullptr, nullptr};
   long long cells = 0;
 };
@@ -565,6 +566,7 @@ GridArgs grid_args(const wf_handle *h) {
     g.pml[a].W = A.W;
     g.pml[a].pitch = A.pitch;
     g.pml[a].prof = A.prof;
+    g.pml[a].full = A.full;
     g.pml[a].psi_cur = A.psi[h->cur];
     g.pml[a].psi_nxt = A.psi[h->cur ^ 1];
     g.pml[a].cells = A.cells;
@@ -1545,7 +1547,13 @@ wf_status wf_set_pml(wf_handle *h, int axis, int T, const float *b, const float 
                         : axis == 1 ? static_cast<long long>(h->nx) * h->nz
                                     : static_cast<long long>(h->nx) * h->ny;
   A.cells = cross * A.pitch;
-  std::vector<float> prof(3 * A.W);
+  const int at = (3 * A.W + 3) / 4 * 4;  // 16-byte aligned
+  std::vector<float> prof(axis == 0 ? at + 3 * n : 3 * A.W);
+  if (axis == 0) {
+    std::copy(b, b + n, prof.begin() + at);
+    std::copy(a, a + n, prof.begin() + at + n);
+    std::copy(ik, ik + n, prof.begin() + at + 2 * n);
+  }
   for (int s = 0; s < A.W; ++s) {
     const int c = s < T ? s : s + (n - A.W);  // slab position -> axis coordinate
     prof[s] = b[c];
@@ -1553,6 +1561,7 @@ wf_status wf_set_pml(wf_handle *h, int axis, int T, const float *b, const float 
     prof[2 * A.W + s] = ik[c];
   }
   WF_CUDA(h, wf::dev_alloc(&A.prof, sizeof(float) * prof.size()));
+  if (axis == 0) A.full = A.prof + at;
   WF_CUDA(h, h2d_sync(A.prof, prof.data(), sizeof(float) * prof.size(), h->stream));
   for (int k = 0; k < 2; ++k) {
     WF_CUDA(h, wf::dev_alloc(&A.psi[k], sizeof(float) * 4 * A.cells));

@@ -31,6 +31,7 @@ struct PmlAxis {
   int pitch;             // x axis: row pitch of the slab array (W rounded up to 4,
                          // so each row starts 16-byte aligned for TMA); y, z: W
   const float *prof;     // [3][W]: b, a, 1/kappa at slab positions
+  const float *full;     // x axis: the same by x coordinate, [3][nx]
   const float *psi_cur;  // [4][cells]: H term 0, H term 1, E term 0, E term 1
   float *psi_nxt;
   long long cells;       // cells per psi component
