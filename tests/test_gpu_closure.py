@@ -287,9 +287,6 @@ def test_weight_gradient_against_float64(n, ci, co, d, h, w, nface):
     """dw adds to what is there; samples whose face is not below nface are left
     out.  Tolerance: FP32 sums of at most n*d*h*w products, error below
     2 * sqrt(terms) * 2^-24 of the sum of magnitudes, plus the final add."""
-    torch = pytest.importorskip("torch")
-    import ctypes as C
-    from wavefront_b200 import lib
     g = torch.Generator(device="cuda").manual_seed(n * 1000 + w)
     x = torch.randn(n, ci, d, h, w, device="cuda", generator=g)
     dz = torch.randn(n, co, d, h, w, device="cuda", generator=g)
@@ -307,7 +304,7 @@ def test_weight_gradient_against_float64(n, ci, co, d, h, w, nface):
             want[f, :, :, t] += torch.einsum("odhw,cdhw->oc", dz[s].double(), win)
             mag[f, :, :, t] += torch.einsum("odhw,cdhw->oc", dz[s].double().abs(), win.abs())
     p = lambda t: C.c_void_p(t.data_ptr())
-    st = lib().wf_nn_conv3d_backward_weight(p(x), p(dz), p(face), p(dw), n, ci, co, d, h, w, nface,
+    st = L.lib().wf_nn_conv3d_backward_weight(p(x), p(dz), p(face), p(dw), n, ci, co, d, h, w, nface,
                                             C.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert st == 0
     tol = 2.0 * (n * d * h * w + 1) ** 0.5 * 2.0 ** -24

@@ -66,17 +66,18 @@ __device__ __forceinline__ void band_du(int al, int ol, int by, int sub, int &d,
 
 // The three bfloat16 parts of 16 FP32 values, as six 16-byte words:
 // out[2 * part + half] holds channels 8 * half .. 8 * half + 7 of `part`.
+// Two values per conversion: the packed form runs on the ALU pipe, the scalar
+// one on the quarter-rate XU pipe, which was 92 % busy in the closure's
+// convolutions (B200, 173 us a layer at 232^2 with scalar conversions).
 __device__ __forceinline__ void split16(float v[16], uint4 out[6]) {
 #pragma unroll
   for (int part = 0; part < 3; ++part) {
     uint32_t q[8];
 #pragma unroll
     for (int c = 0; c < 16; c += 2) {
-      const __nv_bfloat16 h0 = __float2bfloat16_rn(v[c]), h1 = __float2bfloat16_rn(v[c + 1]);
-      q[c / 2] = static_cast<uint32_t>(__bfloat16_as_ushort(h0)) |
-                 (static_cast<uint32_t>(__bfloat16_as_ushort(h1)) << 16);
-      v[c] -= __bfloat162float(h0);
-      v[c + 1] -= __bfloat162float(h1);
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(q[c / 2]) : "f"(v[c + 1]), "f"(v[c]));
+      v[c] -= __uint_as_float(q[c / 2] << 16);
+      v[c + 1] -= __uint_as_float(q[c / 2] & 0xffff0000u);
     }
     out[2 * part] = make_uint4(q[0], q[1], q[2], q[3]);
     out[2 * part + 1] = make_uint4(q[4], q[5], q[6], q[7]);

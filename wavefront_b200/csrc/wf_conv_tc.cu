@@ -1,38 +1,45 @@
 // wf_conv_tc.cu -- the closure network's 3x3x3 convolutions on the sm_100a
 // tensor cores (tcgen05.mma, accumulators in tensor memory), as implicit
-// GEMMs: M = 128 output voxels, N = 16 output channels, K = 16 input channels
-// per tap, 27 taps accumulated into the same tensor-memory tile.
+// GEMMs on FP32 tensors: the training path and the closure's generic one.
 //
 // Numerics.  The weights are bfloat16 (exact operands).  An FP32 activation
 // a is split into three bfloat16 parts, a1 = bf16(a), a2 = bf16(a - a1),
 // a3 = bf16(a - a1 - a2) (each difference exact in FP32), and every part is
-// multiplied by the weight (three MMAs per tap): the operand keeps 24
-// significant bits, like FP32 itself (two parts would keep 16, a relative
-// error up to 2^-16), every product is exact, and the tensor core
-// accumulates in FP32.  Results agree with the FP32 CUDA-core kernels to
-// about 1e-7 relative, not bit for bit (the summation order differs).
+// multiplied by the weight: the operand keeps 24 significant bits, like FP32
+// itself (two parts would keep 16, a relative error up to 2^-16), every
+// product is exact, and the tensor core accumulates in FP32.  Results agree
+// with the FP32 CUDA-core kernels to about 1e-6 relative, not bit for bit
+// (the summation order differs), and with the in-step closure's
+// (wf_closure_fast.cu) operand by operand: the same sums in the same order.
+//
+// One MMA of M 128 x N 144 x K 16 multiplies 128 input voxels of a plane (row
+// offset dy, one part) with the nine taps (dz, dx): it adds to output planes
+// z - 1, z, z + 1, and for each to three dx tiles, which the epilogue shifts
+// by a lane and adds.  No halo columns are needed where the rows are whole
+// (W <= 16: 8 rows x 16 columns a tile); wider tensors use 4 rows x 32 columns
+// of which 30 are kept.
 //
 // Data layout in shared memory (no swizzle, K-major canonical layout: core
 // matrices of 8 rows x 16 bytes):
-//   A  [part 1..3][channel half][plane][row][col] x 8 channels (16 bytes a
-//      voxel): a tile of DT+2 depth planes x 6 rows x 32 columns around the
-//      CTA's DT x 4 x 30 output voxels.  Output voxels (plane p, rows 1..4,
-//      columns 0..31) are 128 consecutive voxels, so one M tile of a plane is
-//      one descriptor, and a tap (dz, dy, dx) only moves its start address by
-//      (dz*192 + dy*32 + dx) voxels.  Columns 0 and 31 are the tile's x halo:
-//      their rows are computed and discarded (30 of every 32 rows are kept).
-//      SBO (8 rows) = 128 bytes; LBO (next 8 channels) = one channel-half array.
-//   B  [tap][channel half][16 output channels][8 input channels]: 512 bytes a
-//      tap, SBO 128, LBO 256.
-// Tensor memory: DT tiles of 128 lanes x 16 FP32 columns (one per plane).
+//   A  [plane][part 1..3][channel half][row][col] x 8 channels (16 bytes a
+//      voxel): up to 6 input planes around the CTA's 4 output planes
+//   B  [dy][channel half][n = 48 j + 16 (dx + 1) + co][8 input channels], row
+//      block j holding dz = 1 - j
+// Tensor memory: 4 planes x 48 FP32 columns.
 //
 // One thread issues all MMAs of the CTA and commits them to an mbarrier;
 // the wait is bounded (a timeout is counted, the epilogue is skipped and the
 // tensor memory is still freed).
+//
+// Measured on B200 (128 samples of 8 x 16 x 16, 16 -> 16 channels): 130 us with
+// one N 16 MMA per tap and part (162 for 2 planes x 4 x 30 outputs, half of
+// them padding at 16 columns); kTcRate now, two CTAs an SM whose load, MMA and
+// epilogue phases overlap.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wf_band.cuh"
 #include "wf_closure.h"
 #include "wf_internal.cuh"
 
@@ -40,21 +47,28 @@ namespace wf {
 
 namespace {
 
-constexpr int kTcDT = 2;            // output depth planes per CTA
-constexpr int kTcParts = 3;         // bfloat16 parts of an FP32 activation
-constexpr int kTcPlanes = kTcDT + 2;
-constexpr int kTcRows = 6;          // 4 output rows + halo
-constexpr int kTcCols = 32;         // 30 output columns + halo
-constexpr int kTcOutRows = 4, kTcOutCols = 30;
-constexpr int kTcVox = kTcPlanes * kTcRows * kTcCols;            // 768
-constexpr int kTcArr = (16 + kTcVox * 16 + 16 + 127) / 128 * 128;  // one [part][half] array, bytes
-constexpr int kTcA = 2 * kTcParts * kTcArr;                        // parts x 2 channel halves
-constexpr int kTcB = 27 * 512;
-constexpr int kTcBar = kTcA + kTcB;
-constexpr int kTcSmem = kTcBar + 16;
-constexpr int kTcThreads = 256;  // 8 warps: two per TMEM lane quarter
-constexpr int kTcCols32 = 32;  // tensor-memory columns allocated (kTcDT x 16, power of two)
-static_assert(kTcDT * 16 <= kTcCols32, "accumulator tiles fit the allocation");
+constexpr int kTcD = 4;                  // output planes per CTA
+constexpr int kTcPlaneN = 48;            // columns of one plane: 3 dx taps x 16 outputs
+constexpr int kTcN = 3 * kTcPlaneN;
+constexpr int kTcWHalf = kTcN * 16;      // one K half of a dy block of weights
+constexpr int kTcWBytes = 3 * 2 * kTcWHalf;
+constexpr int kTcThreads = 256;          // 8 warps: two per TMEM lane quarter
+constexpr int kTcCols = 256;             // tensor-memory columns allocated (kTcD x 48)
+constexpr int kTcZero = 2 * 16 * kTcD * kTcPlaneN;  // zeros: A (128 rows) and B of the clearing MMA
+static_assert(kTcZero >= 4096 && kTcD * kTcPlaneN <= kTcCols, "clearing operands, accumulators");
+
+// COLS 32: 4 output rows x 30 of 32 columns; COLS 16: 8 rows x 16 (W <= 16)
+template <int COLS>
+struct TcL {
+  static constexpr int ROWS = 128 / COLS;          // output rows
+  static constexpr int VOX = (ROWS + 2) * COLS;    // staged voxels of a plane
+  static constexpr int ARR = VOX * 16;             // one [part][half] array
+  static constexpr int PLANE = 6 * ARR;
+  static constexpr int OUTC = COLS == 32 ? 30 : 16;
+  static constexpr int B_OFF = (kTcD + 2) * PLANE, Z_OFF = B_OFF + kTcWBytes, BAR_OFF = Z_OFF + kTcZero;
+  static constexpr int BYTES = BAR_OFF + 16;
+  static_assert(ARR % 128 == 0, "128-byte core-matrix rows");
+};
 
 __device__ unsigned long long g_tc_timeouts;  // bounded-wait expiries (diagnostic)
 
@@ -68,16 +82,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          (static_cast<uint64_t>((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D,
-// M = 128, N = 16.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) |
-                            ((128u >> 4) << 24);
+// kind::f16, BF16 A and B (K-major), FP32 D, M = 128, N = n
+__device__ __forceinline__ uint32_t idesc_n(uint32_t n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
 
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accum) {
+__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                          uint32_t accum) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accum));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -106,34 +121,32 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo_elem, float hi_elem) {
-  const uint32_t a = __bfloat16_as_ushort(__float2bfloat16_rn(lo_elem));
-  const uint32_t b = __bfloat16_as_ushort(__float2bfloat16_rn(hi_elem));
-  return a | (b << 16);
-}
-
 // out[s][co][p] = sum_ci sum_tap W[tap][co][ci] * in[s][ci][p + tap], with
 // W from the bfloat16 weights [F][co][ci][27] (forward) or, for the
 // gradient with respect to the input, [F][ci][co][27] transposed and with
 // the taps flipped (BWD: in = dz with `kin` = co channels, out = ci).
-template <bool BWD>
+template <bool BWD, int COLS>
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_conv_tc(const float *in, const __nv_bfloat16 *w, const int *face, float *z, float *a,
               int kin, int nout, int D, int H, int W, int ndt, int act) {
+  using L = TcL<COLS>;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int s = blockIdx.z / ndt, dt = blockIdx.z % ndt;
-  const int x0 = blockIdx.x * kTcOutCols, y0 = blockIdx.y * kTcOutRows, dp0 = dt * kTcDT;
+  const int x0 = blockIdx.x * L::OUTC - (COLS == 32 ? 1 : 0);  // first staged column
+  const int y0 = blockIdx.y * L::ROWS, dp0 = dt * kTcD;
+  const int np = min(kTcD, D - dp0);                           // output planes
+  const int zlo = max(dp0 - 1, 0), zhi = min(dp0 + np, D - 1);  // input planes
   const int f = face ? face[s] : 0;
   const long long HW = static_cast<long long>(H) * W, P = HW * D;
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar = sbase + kTcBar;
+  const uint32_t bar = sbase + L::BAR_OFF;
 
-  if (warp == 0) {  // tensor memory for the DT accumulator tiles
+  if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&s_tmem)),
-                 "r"(kTcCols32)
+                 "r"(kTcCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -141,13 +154,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     mbar_init(bar, 1);
     mbar_fence_init();
   }
+  for (int i = tid; i < kTcZero / 16; i += kTcThreads)
+    reinterpret_cast<uint4 *>(smem + L::Z_OFF)[i] = make_uint4(0u, 0u, 0u, 0u);
 
-  // B: weights of the sample's face, [tap][half][n 16][k 8] bf16, zero padded.
-  // The face's weights are one contiguous block: copied as it is (16-byte
-  // vectors when it allows) into the A region, which is filled only after,
-  // then rearranged from there.
+  // B: the sample's face's weights, zero padded; the contiguous block is
+  // copied as it is (16-byte vectors when it allows) into the A region, which
+  // is filled only after, and rearranged 16 bytes at a time from there
   {
-    __nv_bfloat16 *sb = reinterpret_cast<__nv_bfloat16 *>(smem + kTcA);
     __nv_bfloat16 *raw = reinterpret_cast<__nv_bfloat16 *>(smem);
     const int wn = BWD ? kin : nout;   // first index of the stored weights (co)
     const int wk = BWD ? nout : kin;   // second (ci)
@@ -161,51 +174,45 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       for (int i = tid; i < nraw; i += kTcThreads) raw[i] = wf[i];
     }
     __syncthreads();
-    for (int i = tid; i < 27 * 256; i += kTcThreads) {
-      const int t = i >> 8, e = i & 255;
-      const int half = e >> 7, n = (e >> 3) & 15, k = half * 8 + (e & 7);
-      __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-      if (n < nout && k < kin) v = BWD ? raw[(k * wk + n) * 27 + (26 - t)] : raw[(n * wk + k) * 27 + t];
-      sb[i] = v;
+    uint4 *sb = reinterpret_cast<uint4 *>(smem + L::B_OFF);
+    for (int i = tid; i < kTcWBytes / 16; i += kTcThreads) {
+      const int n = i % kTcN, half = i / kTcN & 1, r = i / (2 * kTcN);
+      const int o = n % 16, t = (2 - n / kTcPlaneN) * 9 + r * 3 + n / 16 % 3;
+      uint32_t q[4];
+#pragma unroll
+      for (int k2 = 0; k2 < 8; k2 += 2) {
+        uint32_t v = 0u;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int k = half * 8 + k2 + e;
+          if (o < nout && k < kin)
+            v |= static_cast<uint32_t>(__bfloat16_as_ushort(BWD ? raw[(k * wk + o) * 27 + (26 - t)]
+                                                                : raw[(o * wk + k) * 27 + t]))
+                 << (16 * e);
+        }
+        q[k2 / 2] = v;
+      }
+      sb[i] = make_uint4(q[0], q[1], q[2], q[3]);
     }
     __syncthreads();  // the raw copy in the A region is consumed
   }
-  // A: the input tile as three bfloat16 parts, zero outside the tensor
+  // A: the input planes as three bfloat16 parts, zero outside the tensor
   {
-    constexpr int NA = 2 * kTcParts;
-    uint4 *arr[NA];
-#pragma unroll
-    for (int q = 0; q < NA; ++q) arr[q] = reinterpret_cast<uint4 *>(smem + q * kTcArr + 16);
-    if (tid < 2 * NA) {  // guards before and after each array
-      const int q = tid % NA;
-      uint4 *g = tid < NA ? arr[q] - 1 : arr[q] + kTcVox;
-      *g = make_uint4(0u, 0u, 0u, 0u);
-    }
-    const int col = tid & 31;
     const float *src = in + static_cast<long long>(s) * kin * P;
-    for (int pr = tid >> 5; pr < kTcPlanes * kTcRows; pr += kTcThreads / 32) {
-      const int pl = pr / kTcRows, row = pr % kTcRows;
-      const int d = dp0 - 1 + pl, y = y0 - 1 + row, x = x0 - 1 + col;
-      const bool inside = d >= 0 && d < D && y >= 0 && y < H && x >= 0 && x < W;
+    const int nvox = (zhi - zlo + 1) * L::VOX;
+    for (int i = tid; i < nvox; i += kTcThreads) {
+      const int pl = i / L::VOX, vx = i % L::VOX;
+      const int d = zlo + pl, y = y0 - 1 + vx / COLS, x = x0 + vx % COLS;
+      const bool inside = y >= 0 && y < H && x >= 0 && x < W;
       const long long off = d * HW + static_cast<long long>(y) * W + x;
       float v[16];
 #pragma unroll
       for (int c = 0; c < 16; ++c) v[c] = (inside && c < kin) ? __ldg(src + c * P + off) : 0.0f;
-      const int vox = pr * kTcCols + col;
+      uint4 q[6];
+      split16(v, q);
+      uint4 *dst = reinterpret_cast<uint4 *>(smem + pl * L::PLANE) + vx;
 #pragma unroll
-      for (int part = 0; part < kTcParts; ++part) {
-        uint32_t q[8];
-#pragma unroll
-        for (int c = 0; c < 16; c += 2) {  // this part, and the residual left for the next
-          const float h0 = __bfloat162float(__float2bfloat16_rn(v[c]));
-          const float h1 = __bfloat162float(__float2bfloat16_rn(v[c + 1]));
-          q[c / 2] = pack_bf16(h0, h1);
-          v[c] -= h0;
-          v[c + 1] -= h1;
-        }
-        arr[2 * part][vox] = make_uint4(q[0], q[1], q[2], q[3]);
-        arr[2 * part + 1][vox] = make_uint4(q[4], q[5], q[6], q[7]);
-      }
+      for (int k = 0; k < 6; ++k) dst[k * L::VOX] = q[k];
     }
   }
   fence_proxy_async();  // the operands above are read by the tensor core (async proxy)
@@ -213,21 +220,23 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  const int nplanes = min(kTcDT, D - dp0);
 
   if (tid == 0) {
-    const uint32_t b0 = sbase + kTcA;
-    for (int p = 0; p < nplanes; ++p) {
-      const int f0 = ((p + 1) * kTcRows + 1) * kTcCols;  // first output row of plane p
-      for (int t = 0; t < 27; ++t) {
-        const int off = (t / 9 - 1) * kTcRows * kTcCols + ((t / 3) % 3 - 1) * kTcCols + (t % 3 - 1);
-        const uint64_t bd = smem_desc(b0 + t * 512, 256, 128);
+    const uint32_t zb = sbase + L::Z_OFF;
+    umma_bf16(tmem, smem_desc(zb, 2048, 128), smem_desc(zb, kTcZero / 2, 128), idesc_n(kTcD * kTcPlaneN), 0u);
+    const uint64_t ad0 = smem_desc(sbase, L::ARR, 128), bd0 = smem_desc(sbase + L::B_OFF, kTcWHalf, 128);
+    for (int zi = zlo; zi <= zhi; ++zi) {
+      const int lo = max(zi - 1, dp0), hi = min(zi + 1, dp0 + np - 1);  // output planes it feeds
+      const uint32_t id = idesc_n(kTcPlaneN * (hi - lo + 1));
+      const uint32_t d = tmem + kTcPlaneN * (lo - dp0);
+      const uint64_t b0 = bd0 + static_cast<uint64_t>(kTcPlaneN * (lo - zi + 1));  // 16 bytes a row
+      const uint64_t a0 = ad0 + static_cast<uint64_t>((zi - zlo) * (L::PLANE / 16));
 #pragma unroll
-        for (int part = 0; part < kTcParts; ++part) {
-          const uint32_t a_addr = sbase + (2 * part) * kTcArr + 16 + (f0 + off) * 16;
-          umma_bf16(tmem + p * 16, smem_desc(a_addr, kTcArr, 128), bd, (t | part) != 0);
-        }
-      }
+      for (int r = 0; r < 3; ++r)  // dy: output row 0 reads staged row r
+#pragma unroll
+        for (int part = 0; part < 3; ++part)
+          umma_bf16(d, a0 + static_cast<uint64_t>((2 * part * L::ARR + r * COLS * 16) / 16),
+                    b0 + static_cast<uint64_t>(r * 2 * kTcWHalf / 16), id, 1u);
     }
     umma_commit(bar);
   }
@@ -240,14 +249,29 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   if (!done) {
     if (tid == 0) atomicAdd(&g_tc_timeouts, 1ull);
   } else {
-    // epilogue: warp w reads tensor-memory lanes 32(w%4)..+31 of plane w/4's
-    // tile = output rows 32(w%4) + lane: voxel (row 1 + w%4, column lane)
-    const int quarter = warp & 3;
-    const int y = y0 + quarter, x = x0 + lane - 1;
-    const bool keep = lane >= 1 && lane <= kTcOutCols && x < W && y < H;
-    for (int p = warp >> 2; p < nplanes; p += kTcThreads / 128) {
-      float v[16];
-      tmem_ld16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + p * 16, v);
+    // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 of every
+    // second plane from w / 4
+    const int m = 32 * (warp & 3) + lane, c = m % COLS;
+    const int y = y0 + m / COLS, x = x0 + c;
+    const bool keep = x < W && y < H && (COLS == 16 || (c >= 1 && c <= L::OUTC));
+    for (int p = warp >> 2; p < np; p += kTcThreads / 128) {
+      float v[16], e[16];
+      const uint32_t ta = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kTcPlaneN * p;
+      tmem_ld16(ta, v);  // dx = -1: the lane before
+#pragma unroll
+      for (int o = 0; o < 16; ++o) {
+        v[o] = __shfl_up_sync(0xffffffffu, v[o], 1);
+        if (COLS == 16 && c == 0) v[o] = 0.0f;
+      }
+      tmem_ld16(ta + 16, e);  // dx = 0
+#pragma unroll
+      for (int o = 0; o < 16; ++o) v[o] += e[o];
+      tmem_ld16(ta + 32, e);  // dx = +1: the lane after
+#pragma unroll
+      for (int o = 0; o < 16; ++o) {
+        const float u = __shfl_down_sync(0xffffffffu, e[o], 1);
+        v[o] += COLS == 16 && c == 15 ? 0.0f : u;
+      }
       if (keep) {
         const long long q = (dp0 + p) * HW + static_cast<long long>(y) * W + x;
 #pragma unroll
@@ -264,9 +288,23 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcCols)
                  : "memory");
   }
+}
+
+template <bool BWD, int COLS>
+int launch_tc_cols(const float *in, const void *w, const int *face, float *z, float *a, int n, int kin,
+                   int nout, int D, int H, int W, int act, cudaStream_t st) {
+  using L = TcL<COLS>;
+  cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BWD, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       L::BYTES);
+  if (e != cudaSuccess) return e;
+  const int ndt = (D + kTcD - 1) / kTcD;
+  const dim3 grid((W + L::OUTC - 1) / L::OUTC, (H + L::ROWS - 1) / L::ROWS, n * ndt);
+  k_conv_tc<BWD, COLS><<<grid, kTcThreads, L::BYTES, st>>>(in, static_cast<const __nv_bfloat16 *>(w), face,
+                                                           z, a, kin, nout, D, H, W, ndt, act);
+  return cudaGetLastError();
 }
 
 template <bool BWD>
@@ -274,18 +312,9 @@ int launch_tc(const float *in, const void *w, const int *face, float *z, float *
               int nout, int D, int H, int W, int act, cudaStream_t st) {
   if (kin < 1 || kin > 16 || nout < 1 || nout > 16 || n < 1 || D < 1 || H < 1 || W < 1)
     return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kTcSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  const int ndt = (D + kTcDT - 1) / kTcDT;
-  const dim3 grid((W + kTcOutCols - 1) / kTcOutCols, (H + kTcOutRows - 1) / kTcOutRows, n * ndt);
-  k_conv_tc<BWD><<<grid, kTcThreads, kTcSmem, st>>>(in, static_cast<const __nv_bfloat16 *>(w), face,
-                                                     z, a, kin, nout, D, H, W, ndt, act);
-  return cudaGetLastError();
+  // whole rows in one tile where they fit: no halo columns
+  return W <= 16 ? launch_tc_cols<BWD, 16>(in, w, face, z, a, n, kin, nout, D, H, W, act, st)
+                 : launch_tc_cols<BWD, 32>(in, w, face, z, a, n, kin, nout, D, H, W, act, st);
 }
 
 }  // namespace
