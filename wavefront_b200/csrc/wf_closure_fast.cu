@@ -17,12 +17,13 @@
 // a word form the box's 512-byte rows), whose zero fill outside the band is
 // the convolution's zero padding, and its face's pre-arranged weights with one
 // bulk copy.  A tile spans the band's whole depth, so every input plane is
-// loaded once, and one MMA of N = 144 applies the nine taps (dz, dx) of an
-// input plane and row offset dy: three output planes, three dx tiles each
-// (k_conv_fast).  The epilogue shifts and adds the dx tiles, applies GELU and
+// loaded once, and one MMA of N = 48 applies the taps dz = -1, 0, +1 of an
+// input plane to the three output planes it feeds: an M 128 x K 16 MMA costs
+// the same for every N up to 64 (measured on B200), so this does the work of
+// three N = 16 MMAs for the price of one.  The epilogue applies GELU and
 // writes the next layer's input already split; the last layer writes FP32
-// times the face's RMS.  The operands, the FP32 accumulation and the order of
-// every sum are those of k_conv_tc.
+// times the face's RMS.  The operands, the per-output tap order and the FP32
+// accumulation are those of k_conv_tc, so the results equal the FP32 path's.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -43,23 +44,30 @@ constexpr int kFD = 8, kFRows = 6, kFCols = 32, kFOutRows = 4, kFOutCols = 30;
 constexpr int kFPlaneVox = kFRows * kFCols;             // 192 voxels a plane
 constexpr int kFArr = kFPlaneVox * 16;                   // 3072 B: one array of a plane
 constexpr int kFPlaneBytes = 6 * kFArr;                  // 18 432 B: one plane slot
-constexpr int kFPlaneN = 48;                             // columns of one plane: 3 dx taps x 16 outputs
-constexpr int kFN = 3 * kFPlaneN;                        // MMA N: three planes
-constexpr int kFWHalf = kFN * 16;                        // 2304 B: one K half of a weight block
-constexpr int kFWBlock = 2 * kFWHalf;                    // one dy block
-constexpr int kFWBytes = 3 * kFWBlock;                   // 13 824 B: one face's weights
-// Shared memory: [8 plane slots][zero block][2 weight slots][barriers].
-constexpr int kFAOff = 0;
-constexpr int kFZOff = kFAOff + kFD * kFPlaneBytes;
-constexpr int kFZBytes = 4096;                           // zeros: A and B of the clearing MMAs
+constexpr int kFN = 48;                                  // MMA N: three planes x 16 outputs
+constexpr int kFWHalf = kFN * 16;                        // 768 B: one K half of a weight block
+constexpr int kFWBlock = 2 * kFWHalf;                    // one (dy, dx) block
+constexpr int kFWBytes = 9 * kFWBlock;                   // 13 824 B: one face's weights
+// Shared memory: [guard][8 plane slots][guard][zero block][2 weight slots]
+// [barriers].  The corner taps of a plane's first and last output rows read
+// one voxel before or after the slot; those reads only feed the discarded
+// halo lanes, and the guards keep the first and the last slot's inside the
+// allocation.
+constexpr int kFGuard = 128;
+constexpr int kFAOff = kFGuard;
+constexpr int kFZOff = kFAOff + kFD * kFPlaneBytes + kFGuard;
+constexpr int kFZBytes = 4096;                           // A of zeros: clears an accumulator
 constexpr int kFWOff = kFZOff + kFZBytes;
 constexpr int kFBarOff = kFWOff + 2 * kFWBytes;
-// full[8], empty[8], acc_full[8], acc_empty[8], wfull[2], wempty[2], done
-constexpr int kFNumBars = 37;
+// full[8], empty[8], wfull[2], wempty[2], acc_full[2], acc_empty[2], done
+constexpr int kFNumBars = 25;
 constexpr int kFSmem = kFBarOff + kFNumBars * 8 + 128;  // + base alignment slack
 constexpr int kFEpiWarps = 16;                           // 4 lane quarters x 4 plane pairs
 constexpr int kFThreads = 64 + 32 * kFEpiWarps;          // TMA warp, MMA warp, epilogue
-// One accumulator of 8 planes x 48 columns, handed over plane by plane.
+// Two accumulators of 160 columns: planes -1 .. 8 of 16 columns each (the
+// outer two take the products of the first and last plane's out-of-band
+// taps and are never read), 256 columns apart.
+constexpr int kFAccCols = 256;
 constexpr int kFTmemCols = 512;
 static_assert(kFPlaneBytes % 128 == 0 && kFWOff % 128 == 0 && kFSmem <= 227 * 1024,
               "closure conv shared-memory layout");
@@ -80,12 +88,18 @@ __host__ __device__ constexpr uint32_t idesc_n(uint32_t n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// Issued by the lane with `leader` set, in code that the whole warp runs: the
+// operands stay warp-uniform, so they live in the uniform registers the
+// instruction reads.  Inside an `if (lane == 0)` every one of them is moved
+// there first, half a dozen slow moves per MMA on a scheduler that four
+// epilogue warps share: 85-93 cycles per MMA where the unit needs 48 (a layer
+// at 232^2: 267 us so, 177 now; the FP32-output layer 239 and 156).
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accum) {
+                                          uint32_t accum, uint32_t leader) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum));
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accum), "r"(leader));
 }
 
 __device__ __forceinline__ void tc_fence_before() {
@@ -120,9 +134,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+__device__ __forceinline__ void tc_commit(uint32_t bar, uint32_t leader) {
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
+      "r"(leader)
+      : "memory");
 }
 
 
@@ -223,16 +240,16 @@ __global__ void k_face_rms_fold(const float *part, long long stride, int H, int 
   if (threadIdx.x == 0) s[f] = sqrtf(s_sum[0] / static_cast<float>(3 * P)) + 1e-30f;
 }
 
-// Wp[f][dy + 1][half][n 144][k 8] bf16 from W[f][co][ci][27] (zero padded):
-// row n = 48 j + 16 (dx + 1) + co holds the tap with dz = 1 - j, the three
-// planes one input plane feeds and, for each, its three dx taps.
+// Wp[f][r = 3 (dy + 1) + dx + 1][half][n 48][k 8] bf16 from W[f][co][ci][27]
+// (tap (dz + 1) 9 + r, zero padded): rows n = 16 j + co hold the tap with
+// dz = 1 - j, the three planes one input plane feeds.
 __global__ void k_pack_weights(const __nv_bfloat16 *w, int co, int ci, __nv_bfloat16 *wp) {
   const int f = blockIdx.y;
-  constexpr int kPer = 3 * 2 * kFN * 8;
+  constexpr int kPer = 9 * 2 * kFN * 8;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPer; i += gridDim.x * blockDim.x) {
     const int r = i / (2 * kFN * 8), e = i % (2 * kFN * 8);
     const int half = e / (kFN * 8), n = (e / 8) % kFN, k = half * 8 + (e & 7);
-    const int j = n / kFPlaneN, dx = n / 16 % 3, o = n % 16, t = (2 - j) * 9 + r * 3 + dx;
+    const int j = n / 16, o = n % 16, t = (2 - j) * 9 + r;
     __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
     if (o < co && k < ci) v = w[((static_cast<long long>(f) * co + o) * ci + k) * 27 + t];
     wp[static_cast<long long>(f) * kPer + i] = v;
@@ -265,28 +282,19 @@ __device__ __forceinline__ FastTile fast_tile(long long t, int txc, int tyc) {
 //               fill outside the band is the convolution's zero padding), into
 //               eight plane slots, and its face's weights (one bulk copy) into
 //               one of two weight slots;
-//   warp 1      MMA: for each input plane z, each dy and each of the three
-//               bfloat16 parts one MMA of M 128 x N 144 x K 16: the same input
-//               rows feed output planes z - 1, z and z + 1 (N 96 at the band's
-//               ends) through all three dx taps of each, whose weights are
-//               stacked along N.  A plane slot is handed back as soon as its
-//               MMAs are done, a plane of the accumulator as soon as the next
-//               input plane's are;
-//   warps 2-17  epilogue, four warps per plane: tensor memory to registers, the
-//               plane handed back; an output column is the dx = 0 tile's own
-//               lane plus the dx = -1 tile's lane before and the dx = +1 tile's
-//               lane after it; then GELU and the next layer's packed input, or
-//               (LAST) the FP32 correction times s[f].
-// Every wait is bounded; a wait that gives up counts a timeout and ends its
-// role's loop, and the CTA waits (bounded) for its copies and MMAs in flight
-// before it frees tensor memory and exits.
-//
-// Why the dx taps are in N: with one MMA per (dy, dx) the A operand started dx
-// voxels (16 bytes) off its 128-byte core-matrix rows for two taps of three,
-// every such row then took two shared-memory reads, and A was read 27 times a
-// plane: 217 MMAs a tile at 85-93 cycles each (45 when aligned), 0.26 ms a layer
-// at 232^2 x 8 x 6.  Now 72 aligned MMAs of about the same length a tile, and
-// the epilogue's instructions are what bounds it (kFastRate).
+//   warp 1      MMA: one MMA (A of zeros) clears the accumulator, then for each
+//               input plane z, each in-plane tap (dy, dx) and each of the three
+//               bfloat16 parts one MMA of M 128 x N 48 x K 16: the same input
+//               rows feed output planes z + 1, z and z - 1 through the taps
+//               dz = -1, 0, +1, whose weights are stacked along N.  A plane
+//               slot is handed back as soon as its MMAs are done;
+//   warps 2-17  epilogue: tensor memory to registers, the accumulator handed
+//               back, then GELU and the next layer's packed input, or (LAST)
+//               the FP32 correction times s[f].
+// Per output the taps are summed in the order (dz, dy, dx, part), the order
+// of the one-plane form.  Every wait is bounded; a wait that gives up counts
+// a timeout and ends its role's loop, and the CTA waits (bounded) for its
+// copies and MMAs in flight before it frees tensor memory and exits.
 template <bool LAST>
 __global__ void __launch_bounds__(kFThreads, 1)
     k_conv_fast(const __grid_constant__ CUtensorMap tm_in, const __nv_bfloat16 *wp,
@@ -297,7 +305,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   __shared__ uint32_t s_tmem;
   __shared__ int s_pl_issued[kFD], s_pl_used[kFD], s_w_issued[2], s_w_used[2];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform
   const int txc = (W + kFOutCols - 1) / kFOutCols, tyc = (H + kFOutRows - 1) / kFOutRows;
   const long long ntot = 6LL * tyc * txc, t0 = blockIdx.x, tstep = gridDim.x;
   const int ntiles = static_cast<int>((ntot - t0 + tstep - 1) / tstep);
@@ -306,11 +315,11 @@ __global__ void __launch_bounds__(kFThreads, 1)
   const uint32_t a_base = sbase + kFAOff, z_base = sbase + kFZOff, w_base = sbase + kFWOff;
   auto full = [&](int z) { return bars + 8 * z; };
   auto empty = [&](int z) { return bars + 64 + 8 * z; };
-  auto acc_full = [&](int p) { return bars + 128 + 8 * p; };
-  auto acc_empty = [&](int p) { return bars + 192 + 8 * p; };
-  auto wfull = [&](int k) { return bars + 256 + 8 * k; };
-  auto wempty = [&](int k) { return bars + 272 + 8 * k; };
-  const uint32_t done = bars + 288;
+  auto wfull = [&](int k) { return bars + 128 + 8 * k; };
+  auto wempty = [&](int k) { return bars + 144 + 8 * k; };
+  auto acc_full = [&](int k) { return bars + 160 + 8 * k; };
+  auto acc_empty = [&](int k) { return bars + 176 + 8 * k; };
+  const uint32_t done = bars + 192;
 
   for (int i = tid; i < kFZBytes / 16; i += blockDim.x)
     reinterpret_cast<uint4 *>(smem + kFZOff)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -326,14 +335,14 @@ __global__ void __launch_bounds__(kFThreads, 1)
     for (int z = 0; z < kFD; ++z) {
       mbar_init(full(z), 1);
       mbar_init(empty(z), 1);
-      mbar_init(acc_full(z), 1);
-      mbar_init(acc_empty(z), kFEpiWarps / 4);
       s_pl_issued[z] = 0;
       s_pl_used[z] = 0;
     }
     for (int k = 0; k < 2; ++k) {
       mbar_init(wfull(k), 1);
       mbar_init(wempty(k), 1);
+      mbar_init(acc_full(k), 1);
+      mbar_init(acc_empty(k), kFEpiWarps);
       s_w_issued[k] = 0;
       s_w_used[k] = 0;
     }
@@ -343,7 +352,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);  // warp-uniform
   bool ok = true;
 
   if (warp == 0) {
@@ -369,110 +378,91 @@ __global__ void __launch_bounds__(kFThreads, 1)
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     }
   } else if (warp == 1) {
-    constexpr uint32_t kIdClear = idesc_n(kFPlaneN), kIdEnd = idesc_n(2 * kFPlaneN), kIdMid = idesc_n(kFN);
-    const uint64_t zd = smem_desc(z_base, 2048, 128);
+    constexpr uint32_t kIdZero = idesc_n(160), kId48 = idesc_n(kFN);
+    const uint32_t leader = lane == 0 ? 1u : 0u;
     for (int i = 0; i < ntiles && ok; ++i) {
-      const int ws = i & 1;
-      if (lane == 0) {
-        ok = mbar_wait(wfull(ws), (i >> 1) & 1);
-        if (ok) {
-          ++s_w_used[ws];
-          const uint32_t wb = w_base + ws * kFWBytes;
-          // Descriptors of a slot's first row and of the first weight block;
-          // a shifted operand adds its byte offset / 16 to the address field,
-          // which stays below 2^14 (shared memory < 256 KB).
-          const uint64_t ad0 = smem_desc(a_base, kFArr, 128), bd0 = smem_desc(wb, kFWHalf, 128);
-          // the accumulator plane p is free once the tile before was read out;
-          // D = 0 x 0 starts it from zero
-          auto clear = [&](int p) {
-            if (!mbar_wait(acc_empty(p), (i & 1) ^ 1)) return false;
-            tc_fence_after();
-            umma_bf16(tmem + kFPlaneN * p, zd, zd, kIdClear, 0u);
-            return true;
-          };
-          ok = clear(0);
-          for (int z = 0; z < kFD && ok; ++z) {
-            if (z + 1 < kFD) ok = clear(z + 1);
-            if (ok) ok = mbar_wait(full(z), i & 1);
-            if (!ok) break;
-            ++s_pl_used[z];
-            // (the TMA's complete_tx on full(z) orders the plane before these
-            // MMAs, as in a TMA-to-UMMA pipeline: no tcgen05 fence here)
-            // planes z - 1, z, z + 1 inside the band; their weights start at
-            // row 48 when there is no plane z - 1
-            const uint32_t d = tmem + kFPlaneN * (z > 0 ? z - 1 : 0);
-            const uint32_t id = z == 0 || z == kFD - 1 ? kIdEnd : kIdMid;
-            const uint64_t b0 = bd0 + (z == 0 ? kFPlaneN : 0);
+      const int ws = i & 1, acc = i & 1;
+      ok = mbar_wait(acc_empty(acc), ((i >> 1) & 1) ^ 1) && mbar_wait(wfull(ws), (i >> 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      if (lane == 0) ++s_w_used[ws];
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t d0 = tmem + acc * kFAccCols;
+      const uint32_t wb = w_base + ws * kFWBytes;
+      // D = 0 x B: the accumulator's 160 columns start from zero
+      umma_bf16(d0, smem_desc(z_base, 2048, 128), smem_desc(wb, kFWHalf, 128), kIdZero, 0u, leader);
+      // Descriptors of a slot's first row and of the first weight block;
+      // a shifted operand adds its byte offset / 16 to the address field,
+      // which stays below 2^14 (shared memory < 256 KB).
+      const uint64_t ad0 = smem_desc(a_base, kFArr, 128), bd0 = smem_desc(wb, kFWHalf, 128);
+#pragma unroll 1
+      for (int z = 0; z < kFD; ++z) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full(z), i & 1));
+        if (!ok) break;
+        if (lane == 0) ++s_pl_used[z];
+        __syncwarp();
+        // (the TMA's complete_tx on full(z) orders the plane before these
+        // MMAs, as in a TMA-to-UMMA pipeline: no tcgen05 fence here)
+        const uint32_t d = d0 + 16 * z;  // planes z - 1, z, z + 1
+        const uint64_t az = ad0 + static_cast<uint64_t>(z * (kFPlaneBytes / 16));
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {  // dy: output row 0 reads input row r
+        for (int r = 0; r < 9; ++r) {
+          const int row = (r / 3) * kFCols + (r % 3 - 1);  // first A row: output row 1 + dy, dx
+          const uint64_t bd = bd0 + static_cast<uint64_t>(r * kFWBlock / 16);
 #pragma unroll
-              for (int part = 0; part < 3; ++part)
-                umma_bf16(d, ad0 + static_cast<uint64_t>((z * kFPlaneBytes + 2 * part * kFArr + r * kFCols * 16) / 16),
-                          b0 + static_cast<uint64_t>(r * kFWBlock / 16), id, 1u);
-            }
-            tc_commit(empty(z));  // the slot is free once these MMAs are done
-            if (z > 0) tc_commit(acc_full(z - 1));
-          }
-          if (ok) {
-            tc_commit(acc_full(kFD - 1));
-            tc_commit(wempty(ws));
-          }
+          for (int part = 0; part < 3; ++part)
+            umma_bf16(d, az + static_cast<uint64_t>(static_cast<long long>((2 * part) * kFArr / 16 + row)), bd,
+                      kId48, 1u, leader);
         }
+        tc_commit(empty(z), leader);  // the slot is free once these MMAs are done
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (ok) {
+        tc_commit(wempty(ws), leader);
+        tc_commit(acc_full(acc), leader);
+      }
     }
     // every MMA issued completes before the teardown frees tensor memory
-    bool fin = true;
-    if (lane == 0) {
-      tc_commit(done);
-      fin = mbar_wait(done, 0);
-    }
-    if (!(__shfl_sync(0xffffffffu, fin ? 1 : 0, 0) != 0)) ok = false;
+    tc_commit(done, leader);
+    if (!__all_sync(0xffffffffu, mbar_wait(done, 0))) ok = false;
   } else {
-    // warp w reads TMEM lanes 32 (w % 4) ..: output row w % 4 of planes g and
-    // g + 4, g = (w - 2) / 4
+    // warp w reads TMEM lanes 32 (w % 4) ..: output rows 32 (w % 4) + lane of
+    // planes 2 g and 2 g + 1, g = (w - 2) / 4
     const int quarter = warp & 3, g = (warp - 2) >> 2;
-    for (int i = 0; i < ntiles && ok; ++i) {
+    for (int i = 0; i < ntiles; ++i) {
+      const int acc = i & 1;
+      if (lane == 0) ok = mbar_wait(acc_full(acc), (i >> 1) & 1);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) break;
+      tc_fence_after();
       const FastTile tl = fast_tile(t0 + i * tstep, txc, tyc);
+      float v[2][16];
+      const uint32_t ta = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kFAccCols;
+      tmem_ld16(ta + 16 * (2 * g + 1), v[0]);  // plane p at column 16 (p + 1)
+      tmem_ld16(ta + 16 * (2 * g + 2), v[1]);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty(acc));
       const int y = tl.y0 + quarter, x = tl.x0 + lane - 1;
-      const bool keep = lane >= 1 && lane <= kFOutCols && x < W && y < H;
-#pragma unroll 1
-      for (int p = g; p < kFD; p += kFEpiWarps / 4) {
-        if (lane == 0) ok = mbar_wait(acc_full(p), i & 1);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
-        tc_fence_after();
-        float v[16], e[16];
-        const uint32_t ta = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kFPlaneN * p;
-        tmem_ld16(ta, v);  // dx = -1
+      if (lane >= 1 && lane <= kFOutCols && x < W && y < H) {
 #pragma unroll
-        for (int o = 0; o < 16; ++o) v[o] = __shfl_up_sync(0xffffffffu, v[o], 1);
-        tmem_ld16(ta + 16, e);  // dx = 0
-#pragma unroll
-        for (int o = 0; o < 16; ++o) v[o] += e[o];
-        tmem_ld16(ta + 32, e);  // dx = +1
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty(p));
-#pragma unroll
-        for (int o = 0; o < 16; ++o) v[o] += __shfl_down_sync(0xffffffffu, e[o], 1);
-        if (keep) {
-          const long long q = p * HW + static_cast<long long>(y) * W + x;
+        for (int h = 0; h < 2; ++h) {
+          const long long q = (2 * g + h) * HW + static_cast<long long>(y) * W + x;
           if (LAST) {
             const float sf = s[tl.f];
 #pragma unroll
             for (int o = 0; o < 16; ++o)
-              if (o < nout) out_y[(static_cast<long long>(tl.f) * nout + o) * P + q] = v[o] * sf;
+              if (o < nout) out_y[(static_cast<long long>(tl.f) * nout + o) * P + q] = v[h][o] * sf;
           } else {
             if (in_scale) {
               const float m = 1.0f / in_scale[tl.f];  // as face_scale divides: times the reciprocal
 #pragma unroll
-              for (int o = 0; o < 16; ++o) v[o] *= m;
+              for (int o = 0; o < 16; ++o) v[h][o] *= m;
             }
 #pragma unroll
-            for (int o = 0; o < 16; ++o) v[o] = o < nout ? gelu_f(v[o]) : 0.0f;
+            for (int o = 0; o < 16; ++o) v[h][o] = o < nout ? gelu_f(v[h][o]) : 0.0f;
             uint4 wv[6];
-            split16(v, wv);
+            split16(v[h], wv);
             uint4 *op = out_packed + static_cast<long long>(tl.f) * 6 * P + q;
 #pragma unroll
             for (int a = 0; a < 6; ++a) op[a * P] = wv[a];

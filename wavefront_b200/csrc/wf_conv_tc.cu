@@ -12,29 +12,37 @@
 // (the summation order differs), and with the in-step closure's
 // (wf_closure_fast.cu) operand by operand: the same sums in the same order.
 //
-// One MMA of M 128 x N 144 x K 16 multiplies 128 input voxels of a plane (row
-// offset dy, one part) with the nine taps (dz, dx): it adds to output planes
-// z - 1, z, z + 1, and for each to three dx tiles, which the epilogue shifts
-// by a lane and adds.  No halo columns are needed where the rows are whole
-// (W <= 16: 8 rows x 16 columns a tile); wider tensors use 4 rows x 32 columns
-// of which 30 are kept.
+// One MMA of M 128 x N 48 x K 16 multiplies 128 consecutive staged voxels of an
+// input plane, shifted by a tap (dy, dx), with that tap's weights for dz = +1,
+// 0, -1 stacked along N: it adds to output planes z - 1, z, z + 1.  An M 128 x
+// K 16 MMA takes the same 48 cycles for every N up to 64.  Per output the taps
+// are summed in the order (dz, dy, dx, part).
 //
 // Data layout in shared memory (no swizzle, K-major canonical layout: core
 // matrices of 8 rows x 16 bytes):
-//   A  [plane][part 1..3][channel half][row][col] x 8 channels (16 bytes a
-//      voxel): up to 6 input planes around the CTA's 4 output planes
-//   B  [dy][channel half][n = 48 j + 16 (dx + 1) + co][8 input channels], row
-//      block j holding dz = 1 - j
-// Tensor memory: 4 planes x 48 FP32 columns.
+//   A  [plane][part 1..3][channel half][guard, rows of `pitch` voxels, guard] x
+//      8 channels (16 bytes a voxel): up to 6 input planes around the CTA's 4
+//      output planes.  Rows of at most 31 columns are staged whole, with one
+//      zero column after them that is also the halo before the next row
+//      (pitch W + 1, 128 / pitch output rows a tile); wider ones as 30 columns
+//      and both halos (pitch 32, 4 rows).  One M tile is 128 consecutive voxels,
+//      so a tap only moves its start address by dy * pitch + dx voxels.
+//   B  [dy, dx][channel half][n = 16 j + co][8 input channels], row block j
+//      holding dz = 1 - j
+// Tensor memory: 8 planes x 16 FP32 columns, the CTA's 4 output planes in the
+// middle (the outer ones take the products of out-of-tile taps and are never
+// read).
 //
 // One thread issues all MMAs of the CTA and commits them to an mbarrier;
 // the wait is bounded (a timeout is counted, the epilogue is skipped and the
 // tensor memory is still freed).
 //
 // Measured on B200 (128 samples of 8 x 16 x 16, 16 -> 16 channels): 130 us with
-// one N 16 MMA per tap and part (162 for 2 planes x 4 x 30 outputs, half of
-// them padding at 16 columns); kTcRate now, two CTAs an SM whose load, MMA and
-// epilogue phases overlap.
+// one N 16 MMA per tap and part over 2 planes x 4 rows x 32 columns, half of
+// them padding here; 50 us now, two CTAs an SM whose load, MMA and epilogue
+// phases overlap.  (N 144 with the dx taps stacked too took 25 us, but sums in
+// another order: training results then differ from before by more than the
+// FP32 rounding of one order.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -48,27 +56,29 @@ namespace wf {
 namespace {
 
 constexpr int kTcD = 4;                  // output planes per CTA
-constexpr int kTcPlaneN = 48;            // columns of one plane: 3 dx taps x 16 outputs
-constexpr int kTcN = 3 * kTcPlaneN;
-constexpr int kTcWHalf = kTcN * 16;      // one K half of a dy block of weights
-constexpr int kTcWBytes = 3 * 2 * kTcWHalf;
+constexpr int kTcN = 48;                 // MMA N: three planes x 16 outputs
+constexpr int kTcWHalf = kTcN * 16;      // one K half of a (dy, dx) block of weights
+constexpr int kTcWBytes = 9 * 2 * kTcWHalf;
 constexpr int kTcThreads = 256;          // 8 warps: two per TMEM lane quarter
-constexpr int kTcCols = 256;             // tensor-memory columns allocated (kTcD x 48)
-constexpr int kTcZero = 2 * 16 * kTcD * kTcPlaneN;  // zeros: A (128 rows) and B of the clearing MMA
-static_assert(kTcZero >= 4096 && kTcD * kTcPlaneN <= kTcCols, "clearing operands, accumulators");
+constexpr int kTcCols = 16 * (kTcD + 4);  // tensor-memory columns: 128
+constexpr int kTcZero = 4096;            // zeros: A and B of the clearing MMA (128 rows each)
+constexpr int kTcMaxRow = 31;            // rows staged whole up to this width
+static_assert(kTcCols == 128, "a power of two, and the clearing MMA's N");
 
-// COLS 32: 4 output rows x 30 of 32 columns; COLS 16: 8 rows x 16 (W <= 16)
-template <int COLS>
-struct TcL {
-  static constexpr int ROWS = 128 / COLS;          // output rows
-  static constexpr int VOX = (ROWS + 2) * COLS;    // staged voxels of a plane
-  static constexpr int ARR = VOX * 16;             // one [part][half] array
-  static constexpr int PLANE = 6 * ARR;
-  static constexpr int OUTC = COLS == 32 ? 30 : 16;
-  static constexpr int B_OFF = (kTcD + 2) * PLANE, Z_OFF = B_OFF + kTcWBytes, BAR_OFF = Z_OFF + kTcZero;
-  static constexpr int BYTES = BAR_OFF + 16;
-  static_assert(ARR % 128 == 0, "128-byte core-matrix rows");
+// Tile geometry of a width: pitch, output columns and rows, the bytes of one
+// [part][half] array (2 halo rows, 128 voxels and 2 guards) and the total.
+struct TcGeom {
+  int pitch, outc, rows, arr, bytes;
 };
+__host__ __device__ inline TcGeom tc_geom(int W) {
+  TcGeom g;
+  g.pitch = W <= kTcMaxRow ? W + 1 : 32;
+  g.outc = W <= kTcMaxRow ? W : 30;
+  g.rows = 128 / g.pitch;
+  g.arr = (2 * g.pitch + 128 + 2) * 16;
+  g.bytes = kTcWBytes + kTcZero + 16 + (kTcD + 2) * 6 * g.arr;
+  return g;
+}
 
 __device__ unsigned long long g_tc_timeouts;  // bounded-wait expiries (diagnostic)
 
@@ -83,16 +93,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 }
 
 // kind::f16, BF16 A and B (K-major), FP32 D, M = 128, N = n
-__device__ __forceinline__ uint32_t idesc_n(uint32_t n) {
+__host__ __device__ constexpr uint32_t idesc_n(uint32_t n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// Issued by the lane with `leader` set, in code that the whole warp runs (see
+// wf_closure_fast.cu).
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accum) {
+                                          uint32_t accum, uint32_t leader) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum));
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accum), "r"(leader));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -125,23 +137,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 // W from the bfloat16 weights [F][co][ci][27] (forward) or, for the
 // gradient with respect to the input, [F][ci][co][27] transposed and with
 // the taps flipped (BWD: in = dz with `kin` = co channels, out = ci).
-template <bool BWD, int COLS>
+template <bool BWD>
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_conv_tc(const float *in, const __nv_bfloat16 *w, const int *face, float *z, float *a,
               int kin, int nout, int D, int H, int W, int ndt, int act) {
-  using L = TcL<COLS>;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t s_tmem;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const TcGeom G = tc_geom(W);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform
   const int s = blockIdx.z / ndt, dt = blockIdx.z % ndt;
-  const int x0 = blockIdx.x * L::OUTC - (COLS == 32 ? 1 : 0);  // first staged column
-  const int y0 = blockIdx.y * L::ROWS, dp0 = dt * kTcD;
-  const int np = min(kTcD, D - dp0);                           // output planes
+  const bool whole = W <= kTcMaxRow;
+  const int x0 = blockIdx.x * G.outc, y0 = blockIdx.y * G.rows, dp0 = dt * kTcD;
+  const int np = min(kTcD, D - dp0);                            // output planes
   const int zlo = max(dp0 - 1, 0), zhi = min(dp0 + np, D - 1);  // input planes
   const int f = face ? face[s] : 0;
   const long long HW = static_cast<long long>(H) * W, P = HW * D;
-  const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar = sbase + L::BAR_OFF;
+  unsigned char *const sW = smem, *const sZ = smem + kTcWBytes, *const sA = sZ + kTcZero + 16;
+  const uint32_t sbase = smem_u32(smem), bar = sbase + kTcWBytes + kTcZero;
+  const uint32_t a_base = bar + 16;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -155,13 +169,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     mbar_fence_init();
   }
   for (int i = tid; i < kTcZero / 16; i += kTcThreads)
-    reinterpret_cast<uint4 *>(smem + L::Z_OFF)[i] = make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4 *>(sZ)[i] = make_uint4(0u, 0u, 0u, 0u);
 
   // B: the sample's face's weights, zero padded; the contiguous block is
   // copied as it is (16-byte vectors when it allows) into the A region, which
   // is filled only after, and rearranged 16 bytes at a time from there
   {
-    __nv_bfloat16 *raw = reinterpret_cast<__nv_bfloat16 *>(smem);
+    __nv_bfloat16 *raw = reinterpret_cast<__nv_bfloat16 *>(sA);
     const int wn = BWD ? kin : nout;   // first index of the stored weights (co)
     const int wk = BWD ? nout : kin;   // second (ci)
     const int nraw = wn * wk * 27;
@@ -174,10 +188,10 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       for (int i = tid; i < nraw; i += kTcThreads) raw[i] = wf[i];
     }
     __syncthreads();
-    uint4 *sb = reinterpret_cast<uint4 *>(smem + L::B_OFF);
+    uint4 *sb = reinterpret_cast<uint4 *>(sW);
     for (int i = tid; i < kTcWBytes / 16; i += kTcThreads) {
       const int n = i % kTcN, half = i / kTcN & 1, r = i / (2 * kTcN);
-      const int o = n % 16, t = (2 - n / kTcPlaneN) * 9 + r * 3 + n / 16 % 3;
+      const int o = n % 16, t = (2 - n / 16) * 9 + r;
       uint32_t q[4];
 #pragma unroll
       for (int k2 = 0; k2 < 8; k2 += 2) {
@@ -196,82 +210,69 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     }
     __syncthreads();  // the raw copy in the A region is consumed
   }
-  // A: the input planes as three bfloat16 parts, zero outside the tensor
+  // A: the input planes as three bfloat16 parts, zero outside the tensor (the
+  // guards, the halos, and the voxels an M tile reads past its last row)
   {
     const float *src = in + static_cast<long long>(s) * kin * P;
-    const int nvox = (zhi - zlo + 1) * L::VOX;
+    const int nv = 2 * G.pitch + 130, nvox = (zhi - zlo + 1) * nv;
     for (int i = tid; i < nvox; i += kTcThreads) {
-      const int pl = i / L::VOX, vx = i % L::VOX;
-      const int d = zlo + pl, y = y0 - 1 + vx / COLS, x = x0 + vx % COLS;
-      const bool inside = y >= 0 && y < H && x >= 0 && x < W;
+      const int pl = i / nv, vx = i % nv - 1;  // -1: the guard before row 0
+      const int row = vx >= 0 ? vx / G.pitch : -1, c = vx - row * G.pitch;
+      const int d = zlo + pl, y = y0 - 1 + row, x = whole ? c : x0 - 1 + c;
+      const bool inside = vx >= 0 && row < G.rows + 2 && y >= 0 && y < H && x >= 0 && x < W;
       const long long off = d * HW + static_cast<long long>(y) * W + x;
       float v[16];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) v[c] = (inside && c < kin) ? __ldg(src + c * P + off) : 0.0f;
+      for (int c16 = 0; c16 < 16; ++c16)
+        v[c16] = (inside && c16 < kin) ? __ldg(src + c16 * P + off) : 0.0f;
       uint4 q[6];
       split16(v, q);
-      uint4 *dst = reinterpret_cast<uint4 *>(smem + pl * L::PLANE) + vx;
+      uint4 *dst = reinterpret_cast<uint4 *>(sA + pl * 6 * G.arr) + vx + 1;
 #pragma unroll
-      for (int k = 0; k < 6; ++k) dst[k * L::VOX] = q[k];
+      for (int k = 0; k < 6; ++k) dst[k * (G.arr / 16)] = q[k];
     }
   }
   fence_proxy_async();  // the operands above are read by the tensor core (async proxy)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
-  if (tid == 0) {
-    const uint32_t zb = sbase + L::Z_OFF;
-    umma_bf16(tmem, smem_desc(zb, 2048, 128), smem_desc(zb, kTcZero / 2, 128), idesc_n(kTcD * kTcPlaneN), 0u);
-    const uint64_t ad0 = smem_desc(sbase, L::ARR, 128), bd0 = smem_desc(sbase + L::B_OFF, kTcWHalf, 128);
+  if (warp == 0) {
+    const uint32_t leader = lane == 0 ? 1u : 0u, zb = sbase + kTcWBytes;
+    umma_bf16(tmem, smem_desc(zb, 2048, 128), smem_desc(zb, 2048, 128), idesc_n(kTcCols), 0u, leader);
+    const uint64_t ad0 = smem_desc(a_base + 16, G.arr, 128), bd0 = smem_desc(sbase, kTcWHalf, 128);
+    const uint64_t part_off = 2 * static_cast<uint64_t>(G.arr / 16);
     for (int zi = zlo; zi <= zhi; ++zi) {
-      const int lo = max(zi - 1, dp0), hi = min(zi + 1, dp0 + np - 1);  // output planes it feeds
-      const uint32_t id = idesc_n(kTcPlaneN * (hi - lo + 1));
-      const uint32_t d = tmem + kTcPlaneN * (lo - dp0);
-      const uint64_t b0 = bd0 + static_cast<uint64_t>(kTcPlaneN * (lo - zi + 1));  // 16 bytes a row
-      const uint64_t a0 = ad0 + static_cast<uint64_t>((zi - zlo) * (L::PLANE / 16));
+      const uint32_t d = tmem + 16 * (zi - dp0 + 1);  // planes zi - 1, zi, zi + 1
+      const uint64_t az = ad0 + static_cast<uint64_t>((zi - zlo) * 6 * (G.arr / 16));
 #pragma unroll
-      for (int r = 0; r < 3; ++r)  // dy: output row 0 reads staged row r
+      for (int r = 0; r < 9; ++r) {
+        // output row 0, shifted by (dy, dx): staged row 1 + dy, a column more or
+        // less (pitch 32: the first staged column is x0 - 1 and dropped)
+        const uint64_t ar = az + static_cast<uint64_t>(static_cast<long long>((r / 3) * G.pitch + r % 3 - 1));
+        const uint64_t bd = bd0 + static_cast<uint64_t>(r * 2 * kTcWHalf / 16);
 #pragma unroll
         for (int part = 0; part < 3; ++part)
-          umma_bf16(d, a0 + static_cast<uint64_t>((2 * part * L::ARR + r * COLS * 16) / 16),
-                    b0 + static_cast<uint64_t>(r * 2 * kTcWHalf / 16), id, 1u);
+          umma_bf16(d, ar + part * part_off, bd, idesc_n(kTcN), 1u, leader);
+      }
     }
-    umma_commit(bar);
+    if (lane == 0) umma_commit(bar);
+    __syncwarp();
   }
-  // warp 0's other lanes wait here, not in the mbarrier's try-wait loop: a
-  // divergent warp alternates between its paths, and lanes suspended in the
-  // try-wait would hold back the lane issuing the MMAs
-  __syncwarp();
   const bool done = mbar_wait(bar, 0);
   tc_fence_after();
   if (!done) {
     if (tid == 0) atomicAdd(&g_tc_timeouts, 1ull);
   } else {
     // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 of every
-    // second plane from w / 4
-    const int m = 32 * (warp & 3) + lane, c = m % COLS;
-    const int y = y0 + m / COLS, x = x0 + c;
-    const bool keep = x < W && y < H && (COLS == 16 || (c >= 1 && c <= L::OUTC));
+    // second plane from w / 4; lane m is staged voxel m of the output rows
+    const int m = 32 * (warp & 3) + lane, row = m / G.pitch, c = m % G.pitch;
+    const int y = y0 + row, x = whole ? c : x0 - 1 + c;
+    const bool keep = row < G.rows && y < H && x < W && (whole || (c >= 1 && c <= G.outc));
     for (int p = warp >> 2; p < np; p += kTcThreads / 128) {
-      float v[16], e[16];
-      const uint32_t ta = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kTcPlaneN * p;
-      tmem_ld16(ta, v);  // dx = -1: the lane before
-#pragma unroll
-      for (int o = 0; o < 16; ++o) {
-        v[o] = __shfl_up_sync(0xffffffffu, v[o], 1);
-        if (COLS == 16 && c == 0) v[o] = 0.0f;
-      }
-      tmem_ld16(ta + 16, e);  // dx = 0
-#pragma unroll
-      for (int o = 0; o < 16; ++o) v[o] += e[o];
-      tmem_ld16(ta + 32, e);  // dx = +1: the lane after
-#pragma unroll
-      for (int o = 0; o < 16; ++o) {
-        const float u = __shfl_down_sync(0xffffffffu, e[o], 1);
-        v[o] += COLS == 16 && c == 15 ? 0.0f : u;
-      }
+      float v[16];
+      tmem_ld16(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 16 * (p + 2), v);
       if (keep) {
         const long long q = (dp0 + p) * HW + static_cast<long long>(y) * W + x;
 #pragma unroll
@@ -293,28 +294,19 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   }
 }
 
-template <bool BWD, int COLS>
-int launch_tc_cols(const float *in, const void *w, const int *face, float *z, float *a, int n, int kin,
-                   int nout, int D, int H, int W, int act, cudaStream_t st) {
-  using L = TcL<COLS>;
-  cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BWD, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       L::BYTES);
-  if (e != cudaSuccess) return e;
-  const int ndt = (D + kTcD - 1) / kTcD;
-  const dim3 grid((W + L::OUTC - 1) / L::OUTC, (H + L::ROWS - 1) / L::ROWS, n * ndt);
-  k_conv_tc<BWD, COLS><<<grid, kTcThreads, L::BYTES, st>>>(in, static_cast<const __nv_bfloat16 *>(w), face,
-                                                           z, a, kin, nout, D, H, W, ndt, act);
-  return cudaGetLastError();
-}
-
 template <bool BWD>
 int launch_tc(const float *in, const void *w, const int *face, float *z, float *a, int n, int kin,
               int nout, int D, int H, int W, int act, cudaStream_t st) {
   if (kin < 1 || kin > 16 || nout < 1 || nout > 16 || n < 1 || D < 1 || H < 1 || W < 1)
     return cudaErrorInvalidValue;
-  // whole rows in one tile where they fit: no halo columns
-  return W <= 16 ? launch_tc_cols<BWD, 16>(in, w, face, z, a, n, kin, nout, D, H, W, act, st)
-                 : launch_tc_cols<BWD, 32>(in, w, face, z, a, n, kin, nout, D, H, W, act, st);
+  const TcGeom G = tc_geom(W);
+  cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, G.bytes);
+  if (e != cudaSuccess) return e;
+  const int ndt = (D + kTcD - 1) / kTcD;
+  const dim3 grid((W + G.outc - 1) / G.outc, (H + G.rows - 1) / G.rows, n * ndt);
+  k_conv_tc<BWD><<<grid, kTcThreads, G.bytes, st>>>(in, static_cast<const __nv_bfloat16 *>(w), face, z, a,
+                                                    kin, nout, D, H, W, ndt, act);
+  return cudaGetLastError();
 }
 
 }  // namespace
