@@ -303,16 +303,6 @@ __device__ __forceinline__ void brick_h(const GridArgs &g, const ST *e, ST *hb, 
   }
 }
 
-// One stored value in field units.
-template <typename ST>
-__device__ __forceinline__ float stored_get(const ST *p, float su) {
-  using SD = Store<ST>;
-  if constexpr (SD::k16)
-    return __fmul_rn(SD::dec_lo(*reinterpret_cast<const unsigned short *>(p)), su);
-  else
-    return *p;
-}
-
 // The wrapped cells of the periodic axes, where the boxes hold zeros: E on
 // every face the brick shares with the domain's, H on the -x, -y, -z ones.
 __device__ __forceinline__ void patch_periodic(const GridArgs &g, float *sE, float *sH, int x0, int y0,
@@ -360,8 +350,29 @@ __device__ __forceinline__ void patch_periodic(const GridArgs &g, float *sE, flo
   }
 }
 
+// A brick's own sources (their cells, components and this step's values) and
+// probes (cells and components, then samples): lists of hits by list index.
+struct BrickTailSmem {
+  unsigned src, prb;  // bit k: source / probe k has a cell in the brick
+  struct Src {
+    int comp, mode, x, y, z;
+    float v;
+  } s[kBrickTailMax];
+  int4 p[kBrickTailMax];  // comp, x, y, z
+  float raw[kBrickTailMax];
+};
+
+// Programmatic dependent launch: a brick launch may start while the step
+// before is still running and waits here, its barrier and coordinates ready,
+// until that step's results are visible; then it lets the next one start.
+// (A launch without the attribute passes straight through.)
+__device__ __forceinline__ void wait_previous_step() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // One brick.  smem: BrickL<ST>::BYTES, 128-byte aligned.
-template <bool FMA, bool PML, bool XS, typename ST>
+template <bool FMA, bool PML, bool XS, bool TAIL, typename ST>
 __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtensorMap *tmH,
                                            const BrickArgs &a, unsigned char *smem, int x0, int y0,
                                            int z0) {
@@ -370,39 +381,26 @@ __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtenso
   constexpr bool U = SD::k16;
   const GridArgs &g = a.g;
   __shared__ uint64_t s_bar;
-  __shared__ unsigned s_src, s_prb, s_max[2];
+  __shared__ unsigned s_max[2];
+  __shared__ typename std::conditional<TAIL, BrickTailSmem, int>::type s_tail;
+  (void)s_tail;
   const int tid = threadIdx.x;
   ST *sE = reinterpret_cast<ST *>(smem), *sH = reinterpret_cast<ST *>(smem + L::H_OFF);
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const long long N = g.N;
   if (tid == 0) {
     const uint32_t bar = smem_u32(&s_bar);
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmE)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmH)) : "memory");
     mbar_init(bar, 1);
     mbar_fence_init();
+    s_max[0] = s_max[1] = 0u;
+    wait_previous_step();
     // (a nonzero test_extra_tx leaves the phase incomplete after the copies
     // have landed, so the bounded wait runs out: the timeout path, tested)
     mbar_expect_tx(bar, L::E_BYTES + L::H_BYTES + static_cast<uint32_t>(a.test_extra_tx));
     tma_load_4d(smem_u32(sE), tmE, x0 - L::PAD, y0 - 1, z0 - 1, 0, bar);
     tma_load_4d(smem_u32(sH), tmH, x0 - L::PAD, y0 - 1, z0 - 1, 3, bar);
-    s_max[0] = s_max[1] = 0u;
-  }
-  // sources and probes with a cell in this brick (at most 32 of each)
-  if (a.tail.on && tid >= 64 && tid < 128) {
-    const int i = tid & 31;
-    bool hit = false;
-    if (tid < 96) {
-      if (i < a.tail.nsrc) {
-        const SrcDev &q = a.tail.src[i];
-        hit = q.x >= x0 && q.x < x0 + kBrickX &&
-              (q.mode != 0 || (q.y >= y0 && q.y < y0 + kBrickY && q.z >= z0 && q.z < z0 + kBrickZ));
-      }
-    } else if (i < a.tail.nprobe) {
-      const ProbeDev &q = a.tail.probe[i];
-      hit = q.x >= x0 && q.x < x0 + kBrickX && q.y >= y0 && q.y < y0 + kBrickY && q.z >= z0 &&
-            q.z < z0 + kBrickZ;
-    }
-    const unsigned k = __ballot_sync(0xffffffffu, hit);
-    if (i == 0) (tid < 96 ? s_src : s_prb) = k;
   }
 
   // CPML axes the brick's cells or its -x, -y, -z faces meet
@@ -452,6 +450,46 @@ __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtenso
   const unsigned cell = static_cast<unsigned>((z * ny + y) * nx + x);
   ST *const nxt = reinterpret_cast<ST *>(g.nxt);
   in = in && idx_ok(g.err, static_cast<long long>(cell) + (role == 3 ? 0 : 3), N);
+  // sources and probes with a cell in this brick: the first -x warp looks at
+  // the sources, the first -y warp at the probes, and the sources' values are
+  // loaded while the boxes arrive
+  if constexpr (TAIL) {
+    const int li = tid & 31;
+    const bool src_warp = role == 3 && ht - kZh < 32;
+    bool hit = false;
+    if (src_warp) {
+      if (li < a.tail.nsrc) {
+        const SrcDev &q = a.tail.src[li];
+        s_tail.s[li] = BrickTailSmem::Src{q.comp, q.mode, q.x, q.y, q.z, 0.0f};
+        hit = q.x >= x0 && q.x < x0 + kBrickX &&
+              (q.mode != 0 || (q.y >= y0 && q.y < y0 + kBrickY && q.z >= z0 && q.z < z0 + kBrickZ));
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (li == 0) s_tail.src = m;
+    } else if (role == 1 && ht < 32) {
+      bool at = false;
+      if (li < a.tail.nprobe) {
+        const ProbeDev &q = a.tail.probe[li];
+        s_tail.p[li] = make_int4(q.comp, q.x, q.y, q.z);
+        at = q.x >= x0 && q.x < x0 + kBrickX && q.y >= y0 && q.y < y0 + kBrickY && q.z >= z0 &&
+             q.z < z0 + kBrickZ;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, at);
+      if (li == 0) s_tail.prb = m;
+    }
+    wait_previous_step();
+    const bool first = src_warp && li == 0 && x0 == 0 && y0 == 0 && z0 == 0;
+    if (hit || first) {
+      const long long st = __ldcg(a.tail.step);
+      if (hit) {
+        const SrcDev &q = a.tail.src[li];
+        s_tail.s[li].v = st < q.nvals ? q.vals[st] : 0.0f;
+      }
+      if (first) *a.tail.step_next = st + 1;
+    }
+  } else {
+    wait_previous_step();
+  }
   uchar4 id = make_uchar4(0, 0, 0, 0);
   if (in) {
     const uint8_t *m = g.mat + static_cast<unsigned>((z * ny + y) * g.mat_pitch + x);
@@ -668,50 +706,55 @@ __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtenso
   }
 
   // ---- sources in list order, then probes (src/engine.rs:769-782) ----
-  if (!a.tail.on) return;
-  if (s_src | s_prb) {  // (written before the first barrier)
-    const long long st = *a.tail.step;
-    __syncthreads();  // the brick's new fields are visible to its CTA
-    for (unsigned m = s_src; m; m &= m - 1) {
-      const SrcDev q = a.tail.src[__ffs(m) - 1];
-      const float v = st < q.nvals ? q.vals[st] : 0.0f;
-      if constexpr (!U) {
-        if (q.mode == 0) {
-          const long long i = q.comp * N + (static_cast<long long>(q.z) * ny + q.y) * nx + q.x;
-          if (tid == 0 && idx_ok(g.err, i, 6 * N)) g.nxt[i] = __fadd_rn(g.nxt[i], v);
-        } else if (tid < kBrickY * kBrickZ) {
-          const long long i =
-              q.comp * N + (static_cast<long long>(z0 + (tid >> 3)) * ny + y0 + (tid & 7)) * nx + q.x;
-          if (idx_ok(g.err, i, 6 * N)) g.nxt[i] = v;
+  if constexpr (TAIL) {
+    const unsigned mprb = s_tail.prb;
+    if (s_tail.src | mprb) {
+      if (role == 0 && in) {  // by the cell's own thread, on what it just stored
+        for (unsigned m = s_tail.src; m; m &= m - 1) {
+          const BrickTailSmem::Src s = s_tail.s[__ffs(m) - 1];
+          if (s.x < x || s.x > x + 3 || (s.mode == 0 && (s.y != y || s.z != z))) continue;
+          float *f = g.nxt + s.comp * N + cell + (s.x - x);
+          if (idx_ok(g.err, s.comp * N + cell + (s.x - x), 6 * N))
+            *f = s.mode == 0 ? __fadd_rn(*f, s.v) : s.v;
+        }
+        for (unsigned m = mprb; m; m &= m - 1) {
+          const int4 s = s_tail.p[__ffs(m) - 1];
+          if (s.y < x || s.y > x + 3 || s.z != y || s.w != z) continue;
+          if (idx_ok(g.err, s.x * N + cell + (s.y - x), 6 * N))
+            s_tail.raw[__ffs(m) - 1] = g.nxt[s.x * N + cell + (s.y - x)];
         }
       }
-      __syncthreads();
-    }
-    if (tid < 32 && ((s_prb >> tid) & 1u)) {
-      const ProbeDev q = a.tail.probe[tid];
-      const long long i = q.comp * N + (static_cast<long long>(q.z) * ny + q.y) * nx + q.x;
-      if (idx_ok(g.err, i, 6 * N)) {
-        const float raw = stored_get<ST>(reinterpret_cast<const ST *>(g.nxt) + i, u.su);
-        if (q.record && st < q.nsteps) q.trace[st] = raw;
-        if (st >= q.first_step && st < q.nsteps) {
-          const double v = static_cast<double>(raw);
-          for (int f = 0; f < q.nfreq; ++f) {
-            q.sc[f] = __dadd_rn(q.sc[f], __dmul_rn(v, q.cos_tab[st * q.nfreq + f]));
-            q.ss[f] = __dadd_rn(q.ss[f], __dmul_rn(v, q.sin_tab[st * q.nfreq + f]));
+      if (mprb) {
+        const bool mine = role == 1 && ht < 32 && (mprb >> ht & 1u);
+        ProbeDev q;
+        long long st = 0;
+        if (mine) {
+          q = a.tail.probe[ht];
+          st = __ldcg(a.tail.step);
+        }
+        __syncthreads();  // the samples
+        if (mine) {
+          const float raw = s_tail.raw[ht];
+          if (q.record && st < q.nsteps) q.trace[st] = raw;
+          if (st >= q.first_step && st < q.nsteps) {
+            const double v = static_cast<double>(raw);
+            for (int f = 0; f < q.nfreq; ++f) {
+              q.sc[f] = __dadd_rn(q.sc[f], __dmul_rn(v, q.cos_tab[st * q.nfreq + f]));
+              q.ss[f] = __dadd_rn(q.ss[f], __dmul_rn(v, q.sin_tab[st * q.nfreq + f]));
+            }
+            q.n[0] += 1ull;
           }
-          q.n[0] += 1ull;
         }
       }
     }
   }
-  if (x0 == 0 && y0 == 0 && z0 == 0 && tid == 0) *a.tail.step_next = *a.tail.step + 1;
 }
 
 // CTA (x + tiles_x * j, z, band): brick (x, 8 band + j, z).  CTAs run x
 // fastest, then 8 rows of bricks in y, then z, then the next band of rows, so
 // that a brick's z neighbour runs within a few MB of traffic of it and only
 // every 8th y face is far away: halo planes and rows come from L2.
-template <bool FMA, bool PML, bool XS, typename ST>
+template <bool FMA, bool PML, bool XS, bool TAIL, typename ST>
 __global__ void __launch_bounds__(kBrickThreads, PML ? 2 : 3)
     k_brick(const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmH,
             const __grid_constant__ BrickArgs a) {
@@ -722,7 +765,7 @@ __global__ void __launch_bounds__(kBrickThreads, PML ? 2 : 3)
   const int y0 = (blockIdx.z * kBrickBand + j) * kBrickY;
   if (y0 >= a.g.ny) return;
   const int x0 = (blockIdx.x - j * a.tiles_x) * kBrickX;
-  brick_body<FMA, PML, XS, ST>(&tmE, &tmH, a, smem, x0, y0, blockIdx.y * kBrickZ);
+  brick_body<FMA, PML, XS, TAIL, ST>(&tmE, &tmH, a, smem, x0, y0, blockIdx.y * kBrickZ);
 }
 
 // Batched step: CTA i computes brick items[i] = (scene, x0, y0, z0).  The
@@ -741,17 +784,30 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
   for (int i = threadIdx.x; i < static_cast<int>(sizeof(BrickArgs) / 4); i += kBrickThreads)
     reinterpret_cast<int *>(&s_args)[i] = __ldg(src + i);
   __syncthreads();
-  brick_body<false, true, XS, float>(&sc->maps[parity].e, &sc->maps[parity].h, s_args, smem, it.y, it.z,
+  brick_body<false, true, XS, false, float>(&sc->maps[parity].e, &sc->maps[parity].h, s_args, smem, it.y, it.z,
                                      it.w);
+}
+
+// Instantiations of a storage type: no CPML; CPML with an x depth that is a
+// multiple of 4; any CPML.  TAIL: FP32 only.
+using BrickFn = void (*)(CUtensorMap, CUtensorMap, BrickArgs);
+
+template <bool FMA, bool TAIL, typename ST>
+BrickFn brick_fn(int variant) {
+  return variant == 0   ? k_brick<FMA, false, false, TAIL, ST>
+         : variant == 1 ? k_brick<FMA, true, false, TAIL, ST>
+                        : k_brick<FMA, true, true, TAIL, ST>;
 }
 
 template <bool FMA, typename ST>
 cudaError_t brick_prepare_t() {
-  const void *fns[] = {(const void *)k_brick<FMA, false, false, ST>,
-                       (const void *)k_brick<FMA, true, false, ST>,
-                       (const void *)k_brick<FMA, true, true, ST>};
-  for (const void *f : fns) {
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, BrickL<ST>::BYTES);
+  for (int v = 0; v < 3; ++v) {
+    cudaError_t e = cudaFuncSetAttribute(brick_fn<FMA, false, ST>(v),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, BrickL<ST>::BYTES);
+    if constexpr (!Store<ST>::k16)
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(brick_fn<FMA, true, ST>(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 BrickL<ST>::BYTES);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -760,16 +816,23 @@ cudaError_t brick_prepare_t() {
 template <bool FMA, typename ST>
 cudaError_t brick_launch_t(const BrickMaps &m, const BrickArgs &a, cudaStream_t s) {
   const int tiles_y = a.g.ny / kBrickY;
-  const dim3 grid(a.tiles_x * std::min(tiles_y, kBrickBand), a.g.nz / kBrickZ,
-                  (tiles_y + kBrickBand - 1) / kBrickBand);
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(a.tiles_x * std::min(tiles_y, kBrickBand), a.g.nz / kBrickZ,
+                   (tiles_y + kBrickBand - 1) / kBrickBand);
+  c.blockDim = dim3(kBrickThreads);
+  c.dynamicSmemBytes = BrickL<ST>::BYTES;
+  c.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &attr;
+  c.numAttrs = 1;
   const int T = a.g.pml[0].T;
-  if (!(T | a.g.pml[1].T | a.g.pml[2].T))
-    k_brick<FMA, false, false, ST><<<grid, kBrickThreads, BrickL<ST>::BYTES, s>>>(m.e, m.h, a);
-  else if (T % 4 == 0)
-    k_brick<FMA, true, false, ST><<<grid, kBrickThreads, BrickL<ST>::BYTES, s>>>(m.e, m.h, a);
-  else
-    k_brick<FMA, true, true, ST><<<grid, kBrickThreads, BrickL<ST>::BYTES, s>>>(m.e, m.h, a);
-  return cudaGetLastError();
+  const int v = !(T | a.g.pml[1].T | a.g.pml[2].T) ? 0 : (T % 4 == 0 ? 1 : 2);
+  BrickFn f = brick_fn<FMA, false, ST>(v);
+  if constexpr (!Store<ST>::k16)
+    if (a.tail.on) f = brick_fn<FMA, true, ST>(v);
+  return cudaLaunchKernelEx(&c, f, m.e, m.h, a);
 }
 
 }  // namespace
