@@ -327,13 +327,42 @@ __global__ void k_next_shifts(TailArgs t, long long next) {
 // 16-bit state from FP32 values, in three passes: slab maxima of the input,
 // the shift they give each slab (from the larger of its E and H maxima),
 // then the encoding (whose maxima remain).
+//
+// One CTA column per (component, slab) folds its values in registers and adds
+// one atomic per CTA: with one atomic per value the 2 * nslab addresses
+// serialised them all (320^3 on B200: 132 ms a pass; 0.2 to 0.6 ms now).
+constexpr int kSlabThreads = 256;
+
+// Calls f(i) for this CTA's share of the values of slab blockIdx.y of component
+// blockIdx.z, and folds the returned magnitudes into slab_max.
+template <typename F>
+__device__ void slab_fold(long long N, int nxy, unsigned *slab_max, F f) {
+  __shared__ unsigned s_m[kSlabThreads / 32];
+  const int c = blockIdx.z, b = blockIdx.y;
+  const long long base = c * N + static_cast<long long>(b) * kSlabPlanes * nxy;
+  const long long cells = static_cast<long long>(kSlabPlanes) * nxy;
+  unsigned m = 0u;
+  for (long long i = static_cast<long long>(blockIdx.x) * kSlabThreads + threadIdx.x; i < cells;
+       i += static_cast<long long>(gridDim.x) * kSlabThreads)
+    m = max(m, f(base + i));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < kSlabThreads / 32) {
+    m = __reduce_max_sync((1u << (kSlabThreads / 32)) - 1u, s_m[threadIdx.x]);
+    if (threadIdx.x == 0 && m) atomicMax(slab_max + 2 * b + (c >= 3), m);
+  }
+}
+
+dim3 slab_grid(long long N, int nxy) {
+  const long long cells = static_cast<long long>(kSlabPlanes) * nxy;
+  const long long nslab = N / cells;
+  const long long per = (cells + 8 * kSlabThreads - 1) / (8 * kSlabThreads);  // 8 values a thread
+  return dim3(static_cast<unsigned>(per < 1024 ? per : 1024), static_cast<unsigned>(nslab), 6);
+}
+
 __global__ void k_slab_max_f32(const float *in, long long N, int nxy, unsigned *slab_max) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= 6 * N) return;
-  const int c = static_cast<int>(i / N);
-  const int b = static_cast<int>((i % N) / nxy) / kSlabPlanes;
-  const unsigned v = __float_as_uint(fabsf(in[i]));
-  if (v) atomicMax(slab_max + 2 * b + (c >= 3), v);
+  slab_fold(N, nxy, slab_max, [&](long long i) { return __float_as_uint(fabsf(in[i])); });
 }
 __global__ void k_shift_from_max(unsigned *slab_max, int *shift, int nslab) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -345,29 +374,23 @@ __global__ void k_shift_from_max(unsigned *slab_max, int *shift, int nslab) {
 }
 __global__ void k_encode(const float *in, void *out, int prec, long long N, int nxy,
                          const int *shift, unsigned *slab_max) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= 6 * N) return;
-  const int c = static_cast<int>(i / N);
-  const int k = 2 * (static_cast<int>((i % N) / nxy) / kSlabPlanes) + (c >= 3);
-  const float d = enc16(out, i, prec, shift[k], in[i]);
-  const unsigned v = __float_as_uint(fabsf(d));
-  if (v) atomicMax(slab_max + k, v);
+  const int sh = shift[2 * blockIdx.y + (blockIdx.z >= 3)];
+  slab_fold(N, nxy, slab_max,
+            [&](long long i) { return __float_as_uint(fabsf(enc16(out, i, prec, sh, in[i]))); });
 }
 __global__ void k_state_max(const void *in, int prec, long long N, int nxy, const int *shift,
                             unsigned *slab_max) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= 6 * N) return;
-  const int c = static_cast<int>(i / N);
-  const int k = 2 * (static_cast<int>((i % N) / nxy) / kSlabPlanes) + (c >= 3);
-  const unsigned v = __float_as_uint(fabsf(dec16(in, i, prec, shift[k])));
-  if (v) atomicMax(slab_max + k, v);
+  const int sh = shift[2 * blockIdx.y + (blockIdx.z >= 3)];
+  slab_fold(N, nxy, slab_max, [&](long long i) { return __float_as_uint(fabsf(dec16(in, i, prec, sh))); });
 }
+// (8 values a thread of one slab and component: no division per value)
 __global__ void k_decode(const void *in, float *out, int prec, long long N, int nxy,
                          const int *shift) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= 6 * N) return;
-  const int c = static_cast<int>(i / N);
-  out[i] = dec16(in, i, prec, shift[2 * (static_cast<int>((i % N) / nxy) / kSlabPlanes) + (c >= 3)]);
+  const int c = blockIdx.z, b = blockIdx.y, sh = shift[2 * b + (c >= 3)];
+  const long long cells = static_cast<long long>(kSlabPlanes) * nxy, base = c * N + b * cells;
+  for (long long i = static_cast<long long>(blockIdx.x) * kSlabThreads + threadIdx.x; i < cells;
+       i += static_cast<long long>(gridDim.x) * kSlabThreads)
+    out[base + i] = dec16(in, base + i, prec, sh);
 }
 
 // SoA (x fastest) <-> FieldBlock order (src/layout.rs:697-755)
@@ -430,14 +453,14 @@ cudaError_t launch_encode_state(const float *in, void *out, int prec, int nx, in
                                 int *shift, unsigned *slab_max, unsigned long long *ovf,
                                 cudaStream_t s) {
   const long long N = static_cast<long long>(nx) * ny * nz;
-  const unsigned blocks = static_cast<unsigned>((6 * N + 255) / 256);
+  const dim3 blocks = slab_grid(N, nx * ny);
   const int nslab = nz / kSlabPlanes;
   cudaError_t e = cudaMemsetAsync(slab_max, 0, sizeof(unsigned) * 2 * nslab, s);
   if (e != cudaSuccess) return e;
-  k_slab_max_f32<<<blocks, 256, 0, s>>>(in, N, nx * ny, slab_max);
+  k_slab_max_f32<<<blocks, kSlabThreads, 0, s>>>(in, N, nx * ny, slab_max);
   k_shift_from_max<<<(nslab + 255) / 256, 256, 0, s>>>(slab_max, shift, nslab);
   (void)ovf;  // encoding a given state saturates nothing it has to report
-  k_encode<<<blocks, 256, 0, s>>>(in, out, prec, N, nx * ny, shift, slab_max);
+  k_encode<<<blocks, kSlabThreads, 0, s>>>(in, out, prec, N, nx * ny, shift, slab_max);
   return cudaGetLastError();
 }
 
@@ -446,16 +469,14 @@ cudaError_t launch_state_max(const void *in, int prec, int nx, int ny, int nz, c
   const long long N = static_cast<long long>(nx) * ny * nz;
   cudaError_t e = cudaMemsetAsync(slab_max, 0, sizeof(unsigned) * 2 * (nz / kSlabPlanes), s);
   if (e != cudaSuccess) return e;
-  k_state_max<<<static_cast<unsigned>((6 * N + 255) / 256), 256, 0, s>>>(in, prec, N, nx * ny,
-                                                                         shift, slab_max);
+  k_state_max<<<slab_grid(N, nx * ny), kSlabThreads, 0, s>>>(in, prec, N, nx * ny, shift, slab_max);
   return cudaGetLastError();
 }
 
 cudaError_t launch_decode_state(const void *in, float *out, int prec, int nx, int ny, int nz,
                                 const int *shift, cudaStream_t s) {
   const long long N = static_cast<long long>(nx) * ny * nz;
-  k_decode<<<static_cast<unsigned>((6 * N + 255) / 256), 256, 0, s>>>(in, out, prec, N, nx * ny,
-                                                                       shift);
+  k_decode<<<slab_grid(N, nx * ny), kSlabThreads, 0, s>>>(in, out, prec, N, nx * ny, shift);
   return cudaGetLastError();
 }
 
