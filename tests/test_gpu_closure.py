@@ -282,7 +282,8 @@ def test_ablation_closure_on_the_thin_layer(trained):
 
 @pytest.mark.parametrize("n,ci,co,d,h,w,nface", [
     (1, 1, 1, 1, 1, 1, 1), (3, 16, 16, 8, 16, 16, 2), (5, 10, 16, 5, 7, 19, 6),
-    (40, 16, 6, 8, 5, 33, 6), (2, 3, 5, 9, 4, 17, 8), (70, 2, 3, 2, 3, 4, 3)])
+    (40, 16, 6, 8, 5, 33, 6), (2, 3, 5, 9, 4, 17, 8), (70, 2, 3, 2, 3, 4, 3),
+    (64, 16, 16, 8, 16, 16, 6), (65, 10, 16, 1, 7, 13, 6), (64, 16, 6, 3, 24, 24, 4), (66, 1, 1, 2, 1, 1, 1)])
 def test_weight_gradient_against_float64(n, ci, co, d, h, w, nface):
     """dw adds to what is there; samples whose face is not below nface are left
     out.  Tolerance: FP32 sums of at most n*d*h*w products, error below

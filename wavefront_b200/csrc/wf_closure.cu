@@ -205,7 +205,7 @@ __global__ void k_conv_bwd_data(const float *dz, const __nv_bfloat16 *w, const i
 // tile's rows between them; the sums meet in global memory once per CTA.
 // Measured on B200 (a training step on 128 samples of 8 x 16 x 16): 4.37 ms, of
 // which the three layers' weight gradients took 0.69 + 1.59 + 1.44 ms with one
-// thread per weight reading both operands from global memory; 1.23 ms now.
+// thread per weight reading both operands from global memory; 145 us a layer now.
 constexpr int kBwD = 4, kBwY = 4, kBwX = 16;         // tile of dz
 constexpr int kBwRow = 20;                           // input row: 18 columns, 16-byte pitch
 constexpr int kBwIn = (kBwD + 2) * (kBwY + 2) * kBwRow + 4;  // one input channel; + 4: channels
@@ -303,6 +303,167 @@ __global__ void __launch_bounds__(kBwThreads, 2)
   float *out = dw + ((static_cast<long long>(f) * co + o) * ci + c) * kTaps;
 #pragma unroll
   for (int t = 0; t < 27; ++t) {
+    atomicAdd(out + t, acc0[t]);
+    if (o + 1 < co) atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+  }
+}
+
+// The same with one CTA per sample, for many samples whose planes fit in shared
+// memory: a thread (one input channel, two output channels, 27 taps) walks all
+// of the sample's voxels in the order (d, y, x), so every sum of a sample is the
+// one sequential chain it has always been.  The input planes d - 1, d, d + 1 and
+// dz's plane d are resident, and with PRE the next ones arrive by cp.async while
+// d is computed.  Two or three threads share the taps of a pair of outputs,
+// which gives every scheduler two warps; 216 FMAs per 4 columns and pair
+// against 22 to 24 shared loads.  B200, 128 samples of 8 x 16 x 16 (three layers):
+// 167 + 180 + 147 us against 435 us in all for the tiles above, which below about
+// 64 samples fill the chip better; taken from there on because a training step
+// then differs from the one before by the order of the atomic adds alone.
+struct BsGeom {
+  int pitch, in_ch, dz_ch;  // input row, floats of a channel's plane (in, dz)
+  int bytes(int ci, int co, bool pre) const {
+    return 4 * ((pre ? 4 : 3) * ci * in_ch + (pre ? 2 : 1) * 2 * ((co + 1) / 2) * dz_ch);
+  }
+};
+// channels start 4 (mod 8) floats apart modulo the 32 banks
+__host__ __device__ inline BsGeom bs_geom(int H, int W) {
+  const int wg = (W + 3) / 4 * 4;
+  BsGeom g;
+  g.pitch = wg + 4;
+  g.in_ch = (H + 2) * g.pitch;
+  g.in_ch += (12 - g.in_ch % 8) % 8;
+  g.dz_ch = H * wg;
+  g.dz_ch += (12 - g.dz_ch % 8) % 8;
+  return g;
+}
+// The nine tap rows (dz, dy) are split between three groups of threads (0-2,
+// 3-5, 6-8), or between two (0-4, 5-8) where three groups of ci * co / 2 threads
+// would not fit in kBsThreads.
+constexpr int kBsThreads = 288;
+
+__device__ __forceinline__ void cp_async4(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// One plane of a thread's sums for the tap rows (dz, dy) R0 .. R1 - 1.
+template <int R0, int R1>
+__device__ __forceinline__ void bs_plane(const float *z0, const float *z1, const float *const v[3], int H,
+                                         int wg, int pitch, float acc0[15], float acc1[15]) {
+  for (int y = 0; y < H; ++y) {
+#pragma unroll 1
+    for (int x = 0; x < wg; x += 4) {
+      const float4 ga = *reinterpret_cast<const float4 *>(z0 + y * wg + x);
+      const float4 gb = *reinterpret_cast<const float4 *>(z1 + y * wg + x);
+      const float g0[4] = {ga.x, ga.y, ga.z, ga.w}, g1[4] = {gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+      for (int r = R0; r < R1; ++r) {
+        const float *w = v[r / 3] + (y + r % 3) * pitch + x;
+        const float4 a = *reinterpret_cast<const float4 *>(w);
+        const float2 b = *reinterpret_cast<const float2 *>(w + 4);
+        const float e[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            acc0[3 * (r - R0) + k] = __fmaf_rn(g0[i], e[i + k], acc0[3 * (r - R0) + k]);
+            acc1[3 * (r - R0) + k] = __fmaf_rn(g1[i], e[i + k], acc1[3 * (r - R0) + k]);
+          }
+      }
+    }
+  }
+}
+
+template <bool PRE>
+__global__ void __launch_bounds__(kBsThreads, 1)
+    k_conv_bwd_weight_seq(const float *in, const float *dz, const int *face, float *dw, int ci, int co,
+                          int D, int H, int W, int nface) {
+  extern __shared__ __align__(16) float s_t[];
+  const int s = blockIdx.x, f = face ? face[s] : 0;
+  if (f < 0 || f >= nface) return;
+  constexpr int NI = PRE ? 4 : 3, NZ = PRE ? 2 : 1;
+  const BsGeom G = bs_geom(H, W);
+  const int tid = threadIdx.x, wg = (W + 3) / 4 * 4, co2 = (co + 1) / 2;
+  const int span = (ci * co2 + 31) / 32 * 32;  // threads of a group: whole warps
+  const bool three = 3 * span <= kBsThreads;
+  const int grp = tid / span, c = (tid % span) % ci, o = 2 * ((tid % span) / ci);
+  const bool active = o < co;
+  const int nin = ci * G.in_ch, ndz = 2 * co2 * G.dz_ch;
+  float *const s_in = s_t, *const s_dz = s_t + NI * nin;
+  const long long HW = static_cast<long long>(H) * W, P = HW * D;
+  const float *src = in + static_cast<long long>(s) * ci * P, *g = dz + static_cast<long long>(s) * co * P;
+  // halos, the columns past W and a missing last channel stay zero
+  for (int i = tid; i < NI * nin + NZ * ndz; i += blockDim.x) s_t[i] = 0.0f;
+  __syncthreads();
+  auto load_in = [&](int d) {  // plane d into its slot (d = D: zeros)
+    float *dst = s_in + (d + 1) % NI * nin;
+    for (int i = tid >> 4; i < ci * H; i += blockDim.x / 16) {
+      const int ch = i / H, y = i % H;
+      for (int x = tid & 15; x < W; x += 16) {
+        float *q = dst + ch * G.in_ch + (y + 1) * G.pitch + 1 + x;
+        if (d < D)
+          cp_async4(q, src + ch * P + d * HW + static_cast<long long>(y) * W + x);
+        else
+          *q = 0.0f;
+      }
+    }
+  };
+  auto load_dz = [&](int d) {
+    float *dst = s_dz + d % NZ * ndz;
+    for (int i = tid >> 4; i < co * H; i += blockDim.x / 16) {
+      const int ch = i / H, y = i % H;
+      for (int x = tid & 15; x < W; x += 16)
+        cp_async4(dst + ch * G.dz_ch + y * wg + x, g + ch * P + d * HW + static_cast<long long>(y) * W + x);
+    }
+  };
+  auto arrived = [&]() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  };
+  float acc0[15], acc1[15];
+#pragma unroll
+  for (int t = 0; t < 15; ++t) acc0[t] = acc1[t] = 0.0f;
+  load_in(0);
+  load_in(1);
+  load_dz(0);
+  arrived();
+  for (int d = 0; d < D; ++d) {
+    if (PRE && d + 1 < D) {
+      load_in(d + 2);
+      load_dz(d + 1);
+    }
+    if (active) {
+      const float *z0 = s_dz + d % NZ * ndz + o * G.dz_ch;
+      const float *v[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = s_in + (d + k) % NI * nin + c * G.in_ch;
+      const float *z1 = z0 + G.dz_ch;
+      if (three) {
+        if (grp == 0) bs_plane<0, 3>(z0, z1, v, H, wg, G.pitch, acc0, acc1);
+        if (grp == 1) bs_plane<3, 6>(z0, z1, v, H, wg, G.pitch, acc0, acc1);
+        if (grp == 2) bs_plane<6, 9>(z0, z1, v, H, wg, G.pitch, acc0, acc1);
+      } else {
+        if (grp == 0) bs_plane<0, 5>(z0, z1, v, H, wg, G.pitch, acc0, acc1);
+        if (grp == 1) bs_plane<5, 9>(z0, z1, v, H, wg, G.pitch, acc0, acc1);
+      }
+    }
+    if (PRE) {
+      arrived();
+    } else if (d + 1 < D) {
+      __syncthreads();  // plane d - 1's slot and dz are free
+      load_in(d + 2);
+      load_dz(d + 1);
+      arrived();
+    }
+  }
+  if (!active) return;
+  const int t0 = grp * (three ? 9 : 15), nt = min(three ? 9 : 15, kTaps - t0);
+  float *out = dw + ((static_cast<long long>(f) * co + o) * ci + c) * kTaps + t0;
+#pragma unroll
+  for (int t = 0; t < 15; ++t) {
+    if (t >= nt) break;
     atomicAdd(out + t, acc0[t]);
     if (o + 1 < co) atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
   }
@@ -565,6 +726,19 @@ int nn_conv_bwd_weight(const float *in, const float *dz, const int *face, float 
                        int co, int D, int H, int W, int nface, void *stream) {
   if (ci > kMaxC || co > kMaxC || nface > 8 || n < 1) return cudaErrorInvalidValue;
   if (ci < 1 || co < 1 || nface < 1 || D < 1 || H < 1 || W < 1) return cudaSuccess;  // nothing to add
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // one CTA per sample where there are enough samples and the planes fit
+  const BsGeom G = bs_geom(H, W);
+  constexpr int kSmemMax = 227 * 1024;
+  if (n >= 64 && H <= 256 && W <= 256 && G.bytes(ci, co, false) <= kSmemMax) {
+    const bool pre = G.bytes(ci, co, true) <= kSmemMax;
+    auto fn = pre ? k_conv_bwd_weight_seq<true> : k_conv_bwd_weight_seq<false>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    if (e != cudaSuccess) return e;
+    const int span = (ci * ((co + 1) / 2) + 31) / 32 * 32;
+    fn<<<n, 3 * span <= kBsThreads ? 3 * span : 2 * span, G.bytes(ci, co, pre), st>>>(in, dz, face, dw, ci, co, D, H, W, nface);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaFuncSetAttribute(k_conv_bwd_weight, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kBwSmem);
   if (e != cudaSuccess) return e;
@@ -577,8 +751,7 @@ int nn_conv_bwd_weight(const float *in, const float *dz, const int *face, float 
                           ((H + kBwY - 1) / kBwY) * ((D + kBwD - 1) / kBwD);
   const long long want = std::max(1, 2 * nsm / nface);
   dim3 grid(static_cast<unsigned>(std::min(want, tiles)), nface);
-  k_conv_bwd_weight<<<grid, kBwThreads, kBwSmem, static_cast<cudaStream_t>(stream)>>>(in, dz, face, dw, n,
-                                                                                      ci, co, D, H, W);
+  k_conv_bwd_weight<<<grid, kBwThreads, kBwSmem, st>>>(in, dz, face, dw, n, ci, co, D, H, W);
   return cudaGetLastError();
 }
 
