@@ -66,9 +66,9 @@ __device__ __forceinline__ void band_du(int al, int ol, int by, int sub, int &d,
 
 // The three bfloat16 parts of 16 FP32 values, as six 16-byte words:
 // out[2 * part + half] holds channels 8 * half .. 8 * half + 7 of `part`.
-// Two values per conversion: the packed form runs on the ALU pipe, the scalar
-// one on the quarter-rate XU pipe, which was 92 % busy in the closure's
-// convolutions (B200, 173 us a layer at 232^2 with scalar conversions).
+// Two values per conversion, in the order they are stored: half the
+// conversions and no packing.  Its time does not show (B200, 173 us a layer of
+// the closure at 232^2 with scalar conversions, 175 with packed ones).
 __device__ __forceinline__ void split16(float v[16], uint4 out[6]) {
 #pragma unroll
   for (int part = 0; part < 3; ++part) {

@@ -725,7 +725,8 @@ int nn_conv_bwd_data(const float *dz, const void *w_bf16, const int *face, float
 int nn_conv_bwd_weight(const float *in, const float *dz, const int *face, float *dw, int n, int ci,
                        int co, int D, int H, int W, int nface, void *stream) {
   if (ci > kMaxC || co > kMaxC || nface > 8 || n < 1) return cudaErrorInvalidValue;
-  if (ci < 1 || co < 1 || nface < 1 || D < 1 || H < 1 || W < 1) return cudaSuccess;  // nothing to add
+  if (ci < 1 || co < 1) return cudaErrorInvalidConfiguration;  // as an empty launch grid
+  if (nface < 1 || D < 1 || H < 1 || W < 1) return cudaSuccess;  // nothing to add
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // one CTA per sample where there are enough samples and the planes fit
   const BsGeom G = bs_geom(H, W);
