@@ -92,6 +92,30 @@ def test_brick_equals_marching_16bit(precision, dims, pml):
     _same(got, want)
 
 
+# Large grids whose x axis has CPML: an interior of marching tiles with bricks
+# around it, for interiors cut by a ragged x extent, by slabs of several depths
+# and open on the axes without CPML.
+@pytest.mark.parametrize("dims,pml,kw", [
+    ((680, 200, 200), (7, 5, 9), {}),
+    ((520, 264, 200), (16, 16, 16), {"arith": "fma", "nsrc": 33}),
+    ((1032, 136, 104), (10, 0, 0), {"sheet": True}),
+    ((360, 200, 264), (7, 5, 9), {"precision": "f16"}),
+    ((328, 264, 200), (4, 0, 12), {"precision": "bf16"}),
+])
+def test_bricks_around_marching_interior(dims, pml, kw):
+    g = wf.DeviceFieldGrid(wf.GridDims(*dims), precision=kw.get("precision", "f32"))
+    for ax, t in enumerate(pml):
+        if t:
+            g.set_pml_axis(ax, t, *(np.ones(2 * t, np.float32),) * 3)
+    assert g.tiling()[0] == 4 and not g.column_tiles  # both kernels
+    g.close()
+    other = dict(kernel="fused", tiling=(4, 24, 3)) if "precision" in kw else dict(kernel="split")
+    want = _grid(dims, seed=7, pml=pml, **other, **kw)
+    got = _grid(dims, "auto", 7, pml, **kw)
+    assert np.abs(want[0]).max() > 0
+    _same(got, want)
+
+
 def test_default_tiling_round_trips_and_marching_stays_selectable():
     g = wf.DeviceFieldGrid(wf.GridDims(64, 64, 64))
     try:

@@ -1,5 +1,5 @@
 // wf_brick_impl.cuh -- the one-shot fused H->E step: one CTA computes one
-// brick of 32 x 8 x 8 cells and exits (wf_brick.cu and wf_brick16.cu
+// brick of 32 x 8 x 4 cells and exits (wf_brick.cu and wf_brick16.cu
 // instantiate it).
 //
 //  * The brick's E (with a one-cell halo) and old H (with the -x, -y and -z
@@ -29,7 +29,9 @@
 //    without), not by the loads: with everything after the boxes skipped the
 //    same grids take half the time.  Halo groups have warps of their own: done
 //    by the main warps in a second pass they cost 15-20 % (128^3: 48).  Four
-//    planes a brick, two or three CTAs an SM, beat eight planes (128^3: 43.6).
+//    planes a brick, two or three CTAs an SM, beat eight planes (128^3: 43.6)
+//    and bricks of 32 x 4 x 4 at three or four CTAs (44.6, 42.4; 256^3 286,
+//    275 for 250) and 32 x 4 x 8 at two (41.0, 260).
 //    Forcing more CTAs an SM spills and loses (64 registers: 64^3 17 us), and
 //    so does a persistent CTA that prefetches its next brick (128^3: 55).
 #pragma once
@@ -372,9 +374,10 @@ __device__ __forceinline__ void wait_previous_step() {
 }
 
 // One brick.  smem: BrickL<ST>::BYTES, 128-byte aligned.
-template <bool FMA, bool PML, bool XS, bool TAIL, typename ST>
+// ARGS: BrickArgs, or without TAIL BrickGrid
+template <bool FMA, bool PML, bool XS, bool TAIL, typename ST, typename ARGS>
 __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtensorMap *tmH,
-                                           const BrickArgs &a, unsigned char *smem, int x0, int y0,
+                                           const ARGS &a, unsigned char *smem, int x0, int y0,
                                            int z0) {
   using L = BrickL<ST>;
   using SD = Store<ST>;
@@ -761,11 +764,29 @@ __global__ void __launch_bounds__(kBrickThreads, PML ? 2 : 3)
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
-  const unsigned j = a.x_magic ? __umulhi(blockIdx.x, a.x_magic) : blockIdx.x;  // / tiles_x
-  const int y0 = (blockIdx.z * kBrickBand + j) * kBrickY;
-  if (y0 >= a.g.ny) return;
-  const int x0 = (blockIdx.x - j * a.tiles_x) * kBrickX;
-  brick_body<FMA, PML, XS, TAIL, ST>(&tmE, &tmH, a, smem, x0, y0, blockIdx.y * kBrickZ);
+  int x0, y0, z0;
+  if (PML && !TAIL && a.shell.n) {  // around an interior of marching tiles
+    int b = 0, first = 0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+      if (static_cast<int>(blockIdx.x) >= a.shell.end[k]) {
+        b = k + 1;
+        first = a.shell.end[k];
+      }
+    const int3 lo = a.shell.lo[b];
+    const unsigned sx = a.shell.nxy[b].x, sy = a.shell.nxy[b].y;
+    const unsigned i = blockIdx.x - first, q = i / sx, z = q / sy;
+    x0 = (lo.x + static_cast<int>(i - q * sx)) * kBrickX;
+    y0 = (lo.y + static_cast<int>(q - z * sy)) * kBrickY;
+    z0 = (lo.z + static_cast<int>(z)) * kBrickZ;
+  } else {
+    const unsigned j = a.x_magic ? __umulhi(blockIdx.x, a.x_magic) : blockIdx.x;  // / tiles_x
+    y0 = (blockIdx.z * kBrickBand + j) * kBrickY;
+    if (y0 >= a.g.ny) return;
+    x0 = (blockIdx.x - j * a.tiles_x) * kBrickX;
+    z0 = blockIdx.y * kBrickZ;
+  }
+  brick_body<FMA, PML, XS, TAIL, ST>(&tmE, &tmH, a, smem, x0, y0, z0);
 }
 
 // Batched step: CTA i computes brick items[i] = (scene, x0, y0, z0).  The
@@ -777,11 +798,11 @@ __global__ void __launch_bounds__(kBrickThreads, 2)
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
-  __shared__ BrickArgs s_args;
+  __shared__ BrickGrid s_args;
   const int4 it = __ldg(items + blockIdx.x);
   const BrickScene *sc = scenes + it.x;
   const int *src = reinterpret_cast<const int *>(&sc->args[parity]);
-  for (int i = threadIdx.x; i < static_cast<int>(sizeof(BrickArgs) / 4); i += kBrickThreads)
+  for (int i = threadIdx.x; i < static_cast<int>(sizeof(BrickGrid) / 4); i += kBrickThreads)
     reinterpret_cast<int *>(&s_args)[i] = __ldg(src + i);
   __syncthreads();
   brick_body<false, true, XS, false, float>(&sc->maps[parity].e, &sc->maps[parity].h, s_args, smem, it.y, it.z,
@@ -817,8 +838,9 @@ template <bool FMA, typename ST>
 cudaError_t brick_launch_t(const BrickMaps &m, const BrickArgs &a, cudaStream_t s) {
   const int tiles_y = a.g.ny / kBrickY;
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3(a.tiles_x * std::min(tiles_y, kBrickBand), a.g.nz / kBrickZ,
-                   (tiles_y + kBrickBand - 1) / kBrickBand);
+  c.gridDim = a.shell.n ? dim3(a.shell.n)
+                        : dim3(a.tiles_x * std::min(tiles_y, kBrickBand), a.g.nz / kBrickZ,
+                               (tiles_y + kBrickBand - 1) / kBrickBand);
   c.blockDim = dim3(kBrickThreads);
   c.dynamicSmemBytes = BrickL<ST>::BYTES;
   c.stream = s;
@@ -826,7 +848,7 @@ cudaError_t brick_launch_t(const BrickMaps &m, const BrickArgs &a, cudaStream_t 
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &attr;
-  c.numAttrs = 1;
+  c.numAttrs = a.shell.n ? 0 : 1;  // a shell launch joins the interior's stream instead
   const int T = a.g.pml[0].T;
   const int v = !(T | a.g.pml[1].T | a.g.pml[2].T) ? 0 : (T % 4 == 0 ? 1 : 2);
   BrickFn f = brick_fn<FMA, false, ST>(v);

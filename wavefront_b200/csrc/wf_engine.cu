@@ -115,6 +115,8 @@ struct wf_handle {
   bool cfg_user_set = false;  // otherwise chosen from the grid at first use
   bool col_user_set = false;  // wf_set_column_tiles was called
   bool brick = false;         // the step runs as bricks (set with the maps)
+  bool mix = false;           // ... around an interior of marching tiles
+  int mix_lo[3] = {}, mix_hi[3] = {};
   wf::BrickMaps brick_map[2];  // per state buffer read
   wf::FusedMaps maps[2];      // per state buffer (the one read by the step)
   int *d_items = nullptr;     // work items grouped by kernel class
@@ -363,6 +365,63 @@ bool is_brick(const FusedConfig &c) {
   return c.ty == wf::kBrickY && c.zchunk == wf::kBrickZ && c.stages == 1;
 }
 
+// Where an automatic step on CPML runs both: the marching tiles' interior
+// class over the cells whose step, halo and warm-up plane meet no slab, cut to
+// whole bricks, and bricks around it.  False where either cannot run or there
+// is no such box.
+struct MixBox {
+  int lo[3], hi[3];
+};
+bool mix_box(const wf_handle *h, MixBox *m) {
+  if (!brick_ok(h) || !marching_ok(h)) return false;
+  const int brick[3] = {wf::kBrickX, wf::kBrickY, wf::kBrickZ};
+  bool pml = false;
+  for (int a = 0; a < 3; ++a) {
+    const int n = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz), T = h->ax[a].T, b = brick[a];
+    pml = pml || T > 0;
+    m->lo[a] = T > 0 ? T / b * b + b : 0;
+    m->hi[a] = T > 0 ? (n - T) / b * b : n;
+    if (m->hi[a] <= m->lo[a]) return false;
+  }
+  return pml;
+}
+
+// CPML cells of the grid, in millions.
+double shell_cells(const wf_handle *h) {
+  const double n = 1e-6 * static_cast<double>(h->N);
+  double inner = n;
+  for (int a = 0; a < 3; ++a) {
+    const int len = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz);
+    inner *= static_cast<double>(len - h->ax[a].W) / len;
+  }
+  return n - inner;
+}
+
+// Interior cells run at 8.4 to 8.9 us per million as marching tiles and 12.6
+// as bricks of the CPML kernel; the shell at 18 to 20 as bricks, while the
+// marching tiles pay most for the x slabs (36 per million cells of their
+// columns; with y and z slabs only there is nothing to gain).  The cheapest
+// by their times on B200, per million cells n, CPML cells s and interior
+// cells i (two launches, a join and a separate tail: 40):
+//   FP32    bricks 12.6 n + 6.9 s, marching 8 n + 22 s + 100,
+//           both 8.4 i + 18.4 (n - i) + 40 (22 where slabs are not aligned)
+//   16-bit  13.9 n, 6.5 n + 22 s + 100, 6.9 i + 19 (n - i) + 40
+// 16 CPML cells: FP32 320^3 464 -> 437 us, 384^3 792 -> 736, 512^3 1735 ->
+// 1583, 1024^3 10448 -> 10292; binary16 320^3 457 -> 382, 512^3 1605 -> 1373.
+// Eight cells: spheres at 512^3 1747 -> 1600; vacuum at 768^3 4155
+// marching and 4361 both, so marching.
+bool use_mix(const wf_handle *h, MixBox *m) {
+  if (h->cfg_user_set || h->col_user_set || h->ax[0].T == 0 || !mix_box(h, m)) return false;
+  const double n = 1e-6 * static_cast<double>(h->N), s = shell_cells(h);
+  const double i = 1e-6 * (m->hi[0] - m->lo[0]) * static_cast<double>(m->hi[1] - m->lo[1]) *
+                   (m->hi[2] - m->lo[2]);
+  const bool b16 = store16(h);
+  const double bricks = b16 ? 13.9 * n : 12.6 * n + 6.9 * s;
+  const double marching = (b16 ? 6.5 : 8.0) * n + 22.0 * s + 100.0;
+  const double outer = b16 ? 19.0 : (h->ax[0].T % 4 ? 22.0 : 18.4);
+  return (b16 ? 6.9 : 8.4) * i + outer * (n - i) + 40.0 < std::min(bricks, marching);
+}
+
 // Whether the step runs as bricks rather than as marching tiles (or, where
 // neither can, as the split pair).  Unless the caller chose a tiling or the
 // column tiles, the cheaper of the two by their times on B200, in
@@ -381,14 +440,11 @@ bool use_brick(const wf_handle *h) {
   if (h->cfg_user_set) return is_brick(h->cfg);
   if (h->col_user_set) return false;
   if (!marching_ok(h)) return true;
+  MixBox m;
+  if (use_mix(h, &m)) return true;
   const double n = 1e-6 * static_cast<double>(h->N);
   if (store16(h)) return n < 86.0;
-  double inner = n;
-  for (int a = 0; a < 3; ++a) {
-    const int len = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz);
-    inner *= static_cast<double>(len - h->ax[a].W) / len;
-  }
-  const double shell = n - inner;
+  const double shell = shell_cells(h);
   return 2.2 * n < (shell > 0.0 ? 100.0 + 4.0 * shell : 4.0);
 }
 
@@ -436,7 +492,7 @@ bool brick_encode(BrickMaps *m, void *fields, int nx, int ny, int nz, int prec) 
   return encode(&m->e, t, 4, fields, dim, str, ebox) && encode(&m->h, t, 4, fields, dim, str, hbox);
 }
 
-void brick_geometry(BrickArgs *a) {
+void brick_geometry(BrickGrid *a) {
   a->tiles_x = (a->g.nx + kBrickX - 1) / kBrickX;
   a->x_magic = static_cast<unsigned>(((1ull << 32) + a->tiles_x - 1) / a->tiles_x);  // 2^32 -> 0
 }
@@ -450,13 +506,15 @@ namespace {
 // longer chunk recomputes the warm-up plane less often; the issue-bound
 // 16-bit kernel gains most from that.
 FusedConfig default_cfg(const wf_handle *h) {
+  MixBox m{{0, 0, 0}, {h->nx, h->ny, h->nz}};
+  if (!use_mix(h, &m)) m = MixBox{{0, 0, 0}, {h->nx, h->ny, h->nz}};
+  const int nx = m.hi[0] - m.lo[0], ny = m.hi[1] - m.lo[1], nz = m.hi[2] - m.lo[2];
   const bool big = h->nz >= 1024;
   if (store16(h)) return FusedConfig{4, big ? 48 : 32, 3};
   // FP32: 24-plane chunks (fewer warm-up planes) while they still give at
   // least four waves of work items at three CTAs per SM, else 12
-  const long long tiles = static_cast<long long>((h->nx + wf::kTileX - 1) / wf::kTileX) *
-                          ((h->ny + 3) / 4);
-  const long long items24 = tiles * ((h->nz + 23) / 24);
+  const long long tiles = static_cast<long long>((nx + wf::kTileX - 1) / wf::kTileX) * ((ny + 3) / 4);
+  const long long items24 = tiles * ((nz + 23) / 24);
   return FusedConfig{4, items24 >= 4LL * 148 * 3 ? 24 : 12, 3};
 }
 
@@ -480,14 +538,20 @@ wf_status build_maps(wf_handle *h, bool allow_cols = true) {
   const cuuint64_t mdim[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)h->nz};
   const cuuint64_t mstr[2] = {(cuuint64_t)h->mat_pitch, (cuuint64_t)h->mat_pitch * h->ny};
   h->brick = use_brick(h);
+  MixBox mix{};
+  h->mix = h->brick && use_mix(h, &mix);
+  std::copy(std::begin(mix.lo), std::end(mix.lo), h->mix_lo);
+  std::copy(std::begin(mix.hi), std::end(mix.hi), h->mix_hi);
   if (h->brick) {
     h->cols = false;
     for (int b = 0; b < 2; ++b)
       if (!wf::brick_encode(&h->brick_map[b], h->fld[b], h->nx, h->ny, h->nz, h->precision))
         return fail(h, WF_ERR_CUDA, "cuTensorMapEncodeTiled(bricks) failed");
     WF_CUDA(h, wf::brick_prepare(h->precision, h->arith == WF_ARITH_FMA));
-    h->maps_ok = true;
-    return WF_OK;
+    if (!h->mix) {
+      h->maps_ok = true;
+      return WF_OK;
+    }
   }
   const cuuint32_t ebox[4] = {eb[0], eb[1], eb[2], eb[3]};
   const cuuint32_t hbox[4] = {hb[0], hb[1], hb[2], hb[3]};
@@ -519,13 +583,14 @@ wf_status build_maps(wf_handle *h, bool allow_cols = true) {
   // Work lists, one per kernel class (interior first): each class runs the
   // kernel instantiation that carries only the CPML code it needs.
   const FusedArgs a = fused_args(h);
-  const int n_items = a.tiles_x * a.tiles_y * ((h->nz + a.zchunk - 1) / a.zchunk);
+  const int n_items = a.tiles_x * a.tiles_y * ((a.z_hi - a.z_lo + a.zchunk - 1) / a.zchunk);
   std::vector<int> lists[wf::kFusedClassCount];
   for (int i = 0; i < n_items; ++i) lists[wf::fused_item_class(a, h->cfg.ty, i)].push_back(i);
   std::vector<int> all;
   for (int k = 0; k < wf::kFusedClassCount; ++k) {
     h->class_off[k] = static_cast<int>(all.size());
     h->class_n[k] = static_cast<int>(lists[k].size());
+    if (h->mix && k > 0 && h->class_n[k]) return fail(h, WF_ERR_CUDA, "an interior item meets a CPML slab");
     all.insert(all.end(), lists[k].begin(), lists[k].end());
   }
   // column items (low and high x edge, 32-row tiles), one list per class
@@ -694,10 +759,13 @@ TailArgs tail_args(const wf_handle *h) {
 FusedArgs fused_args(const wf_handle *h) {
   FusedArgs a{};
   a.g = grid_args(h);
-  a.x_lo = h->cols ? wf::kColWidth : 0;
-  a.x_hi = h->cols ? h->nx - wf::kColWidth : h->nx;
+  a.x_lo = h->mix ? h->mix_lo[0] : (h->cols ? wf::kColWidth : 0);
+  a.x_hi = h->mix ? h->mix_hi[0] : (h->cols ? h->nx - wf::kColWidth : h->nx);
+  a.y_lo = h->mix ? h->mix_lo[1] : 0;
+  a.z_lo = h->mix ? h->mix_lo[2] : 0;
+  a.z_hi = h->mix ? h->mix_hi[2] : h->nz;
   a.tiles_x = (a.x_hi - a.x_lo + wf::kTileX - 1) / wf::kTileX;
-  a.tiles_y = (h->ny + h->cfg.ty - 1) / h->cfg.ty;
+  a.tiles_y = ((h->mix ? h->mix_hi[1] - h->mix_lo[1] : h->ny) + h->cfg.ty - 1) / h->cfg.ty;
   a.zchunk = h->cfg.zchunk;
   a.has_pml = has_pml(h) ? 1 : 0;
   a.prof_in_smem = (h->ax[0].W <= 64 && h->ax[1].W <= 64 && h->ax[2].W <= 64) ? 1 : 0;
@@ -727,8 +795,34 @@ cudaEvent_t timing_event(wf_handle *h) {
 // Whether a brick step applies the sources and probes itself: few of them,
 // and nothing (the closure) between the step and its sources.
 bool brick_tail(const wf_handle *h) {
-  return h->brick && !store16(h) && !h->closure && (!h->srcs.empty() || !h->probes.empty()) &&
+  return h->brick && !h->mix && !store16(h) && !h->closure && (!h->srcs.empty() || !h->probes.empty()) &&
          h->srcs.size() <= wf::kBrickTailMax && h->probes.size() <= wf::kBrickTailMax;
+}
+
+// The bricks around h's interior box.
+wf::BrickShell mix_shell(const wf_handle *h) {
+  const int b[3] = {wf::kBrickX, wf::kBrickY, wf::kBrickZ}, n[3] = {h->nx, h->ny, h->nz};
+  int lo[3], hi[3], all[3];
+  for (int a = 0; a < 3; ++a) {
+    all[a] = (n[a] + b[a] - 1) / b[a];
+    lo[a] = h->mix_lo[a] / b[a];
+    hi[a] = (h->mix_hi[a] + b[a] - 1) / b[a];
+  }
+  wf::BrickShell s{};
+  int box = 0;
+  auto add = [&](int x0, int x1, int y0, int y1, int z0, int z1) {
+    s.n += (x1 - x0) * (y1 - y0) * (z1 - z0);
+    s.end[box] = s.n;
+    s.lo[box] = make_int3(x0, y0, z0);
+    s.nxy[box++] = make_int2(x1 - x0, y1 - y0);
+  };
+  add(0, all[0], 0, all[1], 0, lo[2]);
+  add(0, all[0], 0, all[1], hi[2], all[2]);
+  add(0, all[0], 0, lo[1], lo[2], hi[2]);
+  add(0, all[0], hi[1], all[1], lo[2], hi[2]);
+  add(0, lo[0], lo[1], hi[1], lo[2], hi[2]);
+  add(hi[0], all[0], lo[1], hi[1], lo[2], hi[2]);
+  return s;
 }
 
 wf::BrickArgs brick_args(const wf_handle *h) {
@@ -745,6 +839,7 @@ wf::BrickArgs brick_args(const wf_handle *h) {
     a.tail.step = h->d_step + h->cur;
     a.tail.step_next = h->d_step + (h->cur ^ 1);
   }
+  if (h->mix) a.shell = mix_shell(h);
   return a;
 }
 
@@ -766,12 +861,25 @@ wf_status enqueue_one(wf_handle *h) {
       wf_status s = build_maps(h);
       if (s != WF_OK) return s;
     }
-    if (!h->brick && !h->fork_ev) {
+    if ((!h->brick || h->mix) && !h->fork_ev) {
       wf_status s = acquire_streams(h);
       if (s != WF_OK) return s;
     }
   }
-  if (use_fused(h) && h->brick) {
+  if (use_fused(h) && h->mix) {
+    // the interior on a side stream, first: its items are the long ones, and
+    // the bricks fill the SMs as they end; disjoint cells of the next state
+    WF_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
+    WF_CUDA(h, cudaStreamWaitEvent(h->side[0], h->fork_ev, 0));
+    e = wf::launch_fused(h->cfg, h->maps[h->cur], fused_args(h), h->d_items, h->class_n[0], 0, fma,
+                         h->side[0]);
+    if (e == cudaSuccess) {
+      WF_CUDA(h, cudaEventRecord(h->join_ev[0], h->side[0]));
+      e = wf::launch_brick(h->brick_map[h->cur], brick_args(h), fma, h->stream);
+      WF_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[0], 0));
+    }
+    if (e == cudaSuccess) h->kernel_launches += 2;
+  } else if (use_fused(h) && h->brick) {
     e = wf::launch_brick(h->brick_map[h->cur], brick_args(h), fma, h->stream);
     if (e == cudaSuccess) h->kernel_launches += 1;
   } else if (use_fused(h)) {
@@ -929,8 +1037,9 @@ wf_status check_device_error(wf_handle *h) {
 
 }  // namespace
 
-// A batch of independent grids stepped by one persistent kernel per step
-// (config: many small scenes of uneven size).  Each grid is an ordinary
+// A batch of independent grids stepped by one launch per step
+// (many small scenes of uneven size): the bricks of every grid, or with a
+// z-march tiling set one persistent launch per CPML class.  Each grid is an ordinary
 // handle on the batch's stream; the batch keeps device tables describing
 // all of them for the batched step kernel and the batched tail.
 struct wf_batch {
@@ -1002,7 +1111,7 @@ wf_status narrow_batch_maps(wf_handle *h, int zchunk, wf::BatchScene *sc) {
   const int cur = h->cur;
   const FusedConfig saved = h->cfg;
   h->cfg = FusedConfig{wf::kColTileRows, zchunk, 3};
-  h->cols = false;
+  h->cols = h->mix = false;
   for (int p = 0; p < 2; ++p) {
     CUtensorMap *m = sc->maps[p];
     std::memset(m, 0, sizeof(CUtensorMap) * 3);
@@ -1080,8 +1189,8 @@ wf_status batch_build(wf_batch *b) {
     for (int p = 0; p < 2; ++p) {
       h->cur = p;
       if (b->brick) {
-        wf::BrickArgs &a = bricks[i].args[p];
-        a = wf::BrickArgs{};
+        wf::BrickGrid &a = bricks[i].args[p];
+        a = wf::BrickGrid{};
         a.g = grid_args(h);
         wf::brick_geometry(&a);
         a.test_extra_tx = h->test_extra_tx;
@@ -1185,9 +1294,10 @@ wf_status batch_build(wf_batch *b) {
   return WF_OK;
 }
 
-// The batched step kernels alone (read parity `cur`): one persistent launch
-// per non-empty class, class 0 on the batch's stream and the others on side
-// streams forked from it and joined back; the classes write disjoint cells.
+// The batched step kernels alone (read parity `cur`): one launch of every
+// brick, or one persistent launch per non-empty class, class 0 on the batch's
+// stream and the others on side streams forked from it and joined back; the
+// classes write disjoint cells.
 wf_status batch_kernel(wf_batch *b, int cur) {
   if (b->brick) {
     WF_CUDA(nullptr, wf::launch_brick_batch(b->d_bricks, b->d_brick_items, b->n_items, cur, b->brick_xs,
@@ -1667,7 +1777,7 @@ wf_status wf_step(wf_handle *h, int nsteps) {
     wf_status s = build_maps(h);
     if (s != WF_OK) return s;
   }
-  if (use_fused(h) && !h->brick && !h->fork_ev) {  // the side streams, outside any capture too
+  if (use_fused(h) && (!h->brick || h->mix) && !h->fork_ev) {  // the side streams, outside any capture too
     wf_status s = acquire_streams(h);
     if (s != WF_OK) return s;
   }
@@ -2013,8 +2123,9 @@ wf_status wf_set_test_stall(wf_handle *h, int extra_bytes) {
 
 wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out) {
   if (!h || !out) return WF_ERR_ARG;
+  MixBox m;  // a mixed step reports its interior's tiling
   const FusedConfig c = h->cfg_user_set ? h->cfg
-                        : use_brick(h)  ? FusedConfig{wf::kBrickY, wf::kBrickZ, 1}
+                        : use_brick(h) && !use_mix(h, &m) ? FusedConfig{wf::kBrickY, wf::kBrickZ, 1}
                                         : default_cfg(h);
   out->tile_rows = c.ty;
   out->z_chunk = c.zchunk;
@@ -2067,8 +2178,11 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   if (st != WF_OK) return st;
   const FusedConfig orig = h->cfg;
   const int orig_cur = h->cur;
-  h->cfg_user_set = true;  // trials and the result are explicit tilings
   std::vector<FusedConfig> cands;
+  // the automatic step first where it mixes bricks and marching tiles (0 rows
+  // here: no tiling names it); every other trial is an explicit tiling
+  MixBox m;
+  if (use_mix(h, &m)) cands.push_back(FusedConfig{0, 0, 0});
   if (brick_ok(h)) cands.push_back(FusedConfig{wf::kBrickY, wf::kBrickZ, 1});
   const int tys[] = {4, 8, 16};
   const int stg[] = {3, 4};
@@ -2091,6 +2205,7 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   probes.swap(h->probes);
   for (const FusedConfig &c : cands) {
     h->cfg = c;
+    h->cfg_user_set = c.ty > 0;
     h->maps_ok = false;
     if (enqueue_one(h) != WF_OK) continue;  // warm-up and attribute set
     cudaEventRecord(e0, h->stream);
@@ -2111,6 +2226,7 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->cfg = bc;
+  h->cfg_user_set = bc.ty > 0;
   h->maps_ok = false;
   drop_graphs(h);
   h->cur = orig_cur;
@@ -2125,11 +2241,7 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
     WF_CUDA(h, memset_sync(h->d_step, 0, 2 * sizeof(long long), h->stream));
     WF_CUDA(h, memset_sync(h->d_ovf, 0, sizeof(unsigned long long), h->stream));
   }
-  if (best) {
-    best->tile_rows = bc.ty;
-    best->z_chunk = bc.zchunk;
-    best->stages = bc.stages;
-  }
+  if (best) wf_get_tiling(h, best);
   if (best_ms) *best_ms = bms;
   return WF_OK;
 }

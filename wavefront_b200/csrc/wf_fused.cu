@@ -22,8 +22,8 @@ static int item_class(const FusedArgs &a, int ty, int item, bool col) {
   const int tyi = (item / a.tiles_x) % a.tiles_y;
   const int zc = item / (a.tiles_x * a.tiles_y);
   const int x0 = col ? (txi == 0 ? 0 : a.g.nx - kColWidth) : a.x_lo + txi * kTileX;
-  const int y0 = tyi * ty;
-  const int k0 = zc * a.zchunk, k1 = std::min(k0 + a.zchunk, a.g.nz);
+  const int y0 = a.y_lo + tyi * ty;
+  const int k0 = a.z_lo + zc * a.zchunk, k1 = std::min(k0 + a.zchunk, a.z_hi);
   const PmlAxis &X = a.g.pml[0], &Y = a.g.pml[1], &Z = a.g.pml[2];
   const int xh = col ? x0 + kColWidth - 1 : std::min(x0 + kTileX, a.x_hi) - 1;
   const int yh = std::min(y0 + ty, a.g.ny) - 1;

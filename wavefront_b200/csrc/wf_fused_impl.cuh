@@ -751,9 +751,9 @@ __global__ void __launch_bounds__(Layout<TY, S, ST, LX>::THREADS, kCtasPerSm<TY,
   // or the high (txi 1) x edge of the grid
   const int x0 = LX == 32 ? a.x_lo + txi * kTileX : (txi == 0 ? 0 : a.g.nx - L::TW);
   const int x_end = LX == 32 ? min(x0 + kTileX, a.x_hi) : x0 + L::TW;
-  const int y0 = tyi * TY;
-  const int k0 = zc * a.zchunk;
-  const int k1 = min(k0 + a.zchunk, a.g.nz);
+  const int y0 = a.y_lo + tyi * TY;
+  const int k0 = a.z_lo + zc * a.zchunk;
+  const int k1 = min(k0 + a.zchunk, a.z_hi);
 
   float4 *s_coef = reinterpret_cast<float4 *>(smem);
   for (int i = threadIdx.x; i < 256; i += blockDim.x) s_coef[i] = a.g.coef[i];

@@ -37,6 +37,9 @@ struct FusedArgs {
   // the x-CPML slabs run as column tiles (tiles_x = 2 in a column launch:
   // the low and the high edge)
   int x_lo, x_hi;
+  // and y from y_lo, z in [z_lo, z_hi): the whole grid, or the CPML-free
+  // interior when bricks compute the rest
+  int y_lo, z_lo, z_hi;
   int has_pml;
   int prof_in_smem;  // every CPML axis has at most 64 slab positions
   int test_extra_tx;  // testing aid: bytes stage 0 expects beyond its copies (0 normally)
@@ -57,12 +60,24 @@ struct BrickTail {
 };
 constexpr int kBrickTailMax = 32;
 
-struct BrickArgs {
+struct BrickGrid {
   GridArgs g;
   int tiles_x;
   unsigned x_magic;   // ceil(2^32 / tiles_x), i / tiles_x as a high product (0: tiles_x is 1)
   int test_extra_tx;  // as in FusedArgs
+};
+// The bricks outside an interior box that the marching tiles compute, as six
+// boxes of bricks: z slabs, y slabs between them, x slabs between those.
+// n = 0: every brick of the grid.
+struct BrickShell {
+  int n;       // bricks
+  int end[6];  // of boxes 0..i
+  int3 lo[6];  // first brick
+  int2 nxy[6]; // extent in x and y
+};
+struct BrickArgs : BrickGrid {
   BrickTail tail;
+  BrickShell shell;
 };
 
 struct BrickMaps {
@@ -71,7 +86,7 @@ struct BrickMaps {
 // Encodes the maps over a state of 6*nx*ny*nz values (16-byte aligned), and
 // fills a->tiles_x and x_magic from a->g (wf_engine.cu).
 bool brick_encode(BrickMaps *m, void *fields, int nx, int ny, int nz, int prec);
-void brick_geometry(BrickArgs *a);
+void brick_geometry(BrickGrid *a);
 // TMA boxes of a brick's E and H
 void brick_boxes(int prec, unsigned e_box[4], unsigned h_box[4]);
 cudaError_t brick_prepare(int prec, bool fma);
@@ -82,7 +97,7 @@ cudaError_t launch_brick(const BrickMaps &m, const BrickArgs &a, bool fma, cudaS
 // depth is not a multiple of 4.
 struct BrickScene {
   BrickMaps maps[2];
-  BrickArgs args[2];
+  BrickGrid args[2];
 };
 cudaError_t brick_batch_prepare();
 cudaError_t launch_brick_batch(const BrickScene *scenes, const int4 *items, int n_items, int parity,

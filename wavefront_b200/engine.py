@@ -427,7 +427,7 @@ def run(grid: DeviceFieldGrid, sources: Sequence, probes: Sequence, config: Engi
 
 
 class DeviceBatch:
-    """Many independent grids stepped together by one persistent kernel per
+    """Many independent grids stepped together by one kernel launch per
     step (wf_batch_*).  grid(i) gives the per-grid handle for setup (scene,
     CPML, sources, probes) and read-back; step() advances every grid."""
 
