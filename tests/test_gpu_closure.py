@@ -310,3 +310,37 @@ def test_weight_gradient_against_float64(n, ci, co, d, h, w, nface):
     assert st == 0
     tol = 2.0 * (n * d * h * w + 1) ** 0.5 * 2.0 ** -24
     assert ((dw.double() - want).abs() <= tol * mag + 1e-30).all()
+
+
+@pytest.mark.parametrize("n", [1, 64])
+def test_weight_gradient_leaves_out_taps_beyond_the_planes(n):
+    """An infinite dz at a corner reaches only the taps whose input is inside
+    the planes, an infinite input only those whose dz is; the other sums stay
+    finite, and equal those of the same call without infinities but for the
+    terms at that voxel (which are left out there by a zero)."""
+    ci, co, d, h, w = 3, 4, 3, 6, 18
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand(n, ci, d, h, w, device="cuda", generator=g) + 0.5
+    dz = torch.rand(n, co, d, h, w, device="cuda", generator=g) + 0.5
+    dz[0, 1, 0, 0, 0] = 0.0
+    x[0, 2, d - 1, h - 1, w - 1] = 0.0
+    p = lambda t: C.c_void_p(t.data_ptr())
+
+    def run():
+        dw = torch.zeros(co, ci, 27, device="cuda")
+        st = L.lib().wf_nn_conv3d_backward_weight(p(x), p(dz), None, p(dw), n, ci, co, d, h, w, 1,
+                                                  C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0
+        return dw.cpu().numpy()
+
+    plain = run()
+    dz[0, 1, 0, 0, 0] = float("inf")
+    x[0, 2, d - 1, h - 1, w - 1] = float("inf")
+    got = run()
+    inside = np.array([t // 9 >= 1 and t // 3 % 3 >= 1 and t % 3 >= 1 for t in range(27)])
+    hit = np.zeros((co, ci, 27), bool)
+    hit[1, :, inside] = True  # input (tap) at or after the first voxel
+    hit[:, 2, inside] = True  # dz (minus tap) at or before the last one
+    assert np.isposinf(got[hit]).all()
+    tol = 2.0 * (n * d * h * w + 1) ** 0.5 * 2.0 ** -24
+    np.testing.assert_allclose(got[~hit], plain[~hit], rtol=tol, atol=0)

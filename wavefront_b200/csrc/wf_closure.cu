@@ -193,6 +193,24 @@ __global__ void k_conv_bwd_data(const float *dz, const __nv_bfloat16 *w, const i
   for (int c = 0; c < ci; ++c) din[(static_cast<long long>(s) * ci + c) * P + p] = acc[c];
 }
 
+// The sum of tap t's products over the voxels [d0,d1) x [y0,y1) x [x0,x1) of
+// one sample's channels, the taps outside the planes left out.  The staged
+// kernels multiply their zero halo instead, which only an infinity or a NaN on
+// the other side turns into something else: a sum that is not finite is taken
+// again here.
+__device__ float bw_checked(const float *v, const float *g, int t, int d0, int d1, int y0, int y1,
+                            int x0, int x1, int D, int H, int W, float sum) {
+  const int od = t / 9 - 1, oy = t / 3 % 3 - 1, ox = t % 3 - 1;
+  for (int d = max(d0, -od); d < min(d1, D - od); ++d)
+    for (int y = max(y0, -oy); y < min(y1, H - oy); ++y) {
+      const float *gr = g + (static_cast<long long>(d) * H + y) * W;
+      const float *vr = v + (static_cast<long long>(d + od) * H + y + oy) * W + ox;
+      for (int x = max(x0, -ox); x < min(x1, W - ox); ++x) sum = __fmaf_rn(gr[x], vr[x], sum);
+    }
+  return sum;
+}
+__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
+
 // dw[face][co][ci][tap] += sum over samples of that face and voxels p of
 // dz[n][co][p] * in[n][ci][p + tap].
 //
@@ -301,10 +319,38 @@ __global__ void __launch_bounds__(kBwThreads, 2)
   }
   if (!any || !active) return;
   float *out = dw + ((static_cast<long long>(f) * co + o) * ci + c) * kTaps;
+  unsigned long long bad = 0;  // bit t: acc0[t], bit 32 + t: acc1[t]
 #pragma unroll
   for (int t = 0; t < 27; ++t) {
-    atomicAdd(out + t, acc0[t]);
-    if (o + 1 < co) atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+    if (not_finite(acc0[t]))
+      bad |= 1ull << t;
+    else
+      atomicAdd(out + t, acc0[t]);
+    if (o + 1 >= co) continue;
+    if (not_finite(acc1[t]))
+      bad |= 1ull << (32 + t);
+    else
+      atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+  }
+  for (; bad; bad &= bad - 1) {
+    const int b = __ffsll(static_cast<long long>(bad)) - 1, t = b & 31, k = b >> 5;
+    float sum = 0.0f;
+    count = 0;
+    for (int s = 0; s < n; ++s) {  // this thread's rows of this CTA's tiles
+      if ((face ? face[s] : 0) != f) continue;
+      const float *v = in + (static_cast<long long>(s) * ci + c) * P;
+      const float *g = dz + (static_cast<long long>(s) * co + o + k) * P;
+      int q = static_cast<int>((blockIdx.x + gridDim.x - count % gridDim.x) % gridDim.x);
+      for (; q < tiles; q += gridDim.x) {
+        const int x0 = q % tx * kBwX, y0 = q / tx % ty * kBwY, d0 = q / (tx * ty) * kBwD;
+        for (int row = part; row < kBwD * kBwY; row += parts) {
+          const int d = d0 + row / kBwY, y = y0 + row % kBwY;
+          if (d < D && y < H) sum = bw_checked(v, g, t, d, d + 1, y, y + 1, x0, min(x0 + kBwX, W), D, H, W, sum);
+        }
+      }
+      count += tiles;
+    }
+    atomicAdd(out + static_cast<long long>(k) * ci * kTaps + t, sum);
   }
 }
 
@@ -461,11 +507,24 @@ __global__ void __launch_bounds__(kBsThreads, 1)
   if (!active) return;
   const int t0 = grp * (three ? 9 : 15), nt = min(three ? 9 : 15, kTaps - t0);
   float *out = dw + ((static_cast<long long>(f) * co + o) * ci + c) * kTaps + t0;
+  unsigned bad = 0;  // bit t: acc0[t], bit 16 + t: acc1[t]
 #pragma unroll
   for (int t = 0; t < 15; ++t) {
     if (t >= nt) break;
-    atomicAdd(out + t, acc0[t]);
-    if (o + 1 < co) atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+    if (not_finite(acc0[t]))
+      bad |= 1u << t;
+    else
+      atomicAdd(out + t, acc0[t]);
+    if (o + 1 >= co) continue;
+    if (not_finite(acc1[t]))
+      bad |= 1u << (16 + t);
+    else
+      atomicAdd(out + static_cast<long long>(ci) * kTaps + t, acc1[t]);
+  }
+  for (; bad; bad &= bad - 1) {
+    const int b = __ffs(bad) - 1, t = b & 15, k = b >> 4;
+    atomicAdd(out + static_cast<long long>(k) * ci * kTaps + t,
+              bw_checked(src + c * P, g + (o + k) * P, t0 + t, 0, D, 0, H, 0, W, D, H, W, 0.0f));
   }
 }
 
