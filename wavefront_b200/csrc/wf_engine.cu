@@ -408,7 +408,7 @@ double shell_cells(const wf_handle *h) {
 //   16-bit  13.9 n, 6.5 n + 22 s + 100, 6.9 i + 19 (n - i) + 40
 // 16 CPML cells: FP32 320^3 464 -> 437 us, 384^3 792 -> 736, 512^3 1735 ->
 // 1583, 1024^3 10448 -> 10292; binary16 320^3 457 -> 382, 512^3 1605 -> 1373.
-// Eight cells: spheres at 512^3 1747 -> 1600; vacuum at 768^3 4155
+// Eight cells, vacuum: 384^3 750 -> 649, 512^3 1394 and 1400, 768^3 4155
 // marching and 4361 both, so marching.
 bool use_mix(const wf_handle *h, MixBox *m) {
   if (h->cfg_user_set || h->col_user_set || h->ax[0].T == 0 || !mix_box(h, m)) return false;
