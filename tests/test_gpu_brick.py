@@ -128,3 +128,61 @@ def test_default_tiling_round_trips_and_marching_stays_selectable():
         g.sync()
     finally:
         g.close()
+
+
+# CPML depths on x that leave every group straddling the slab: at depth 1 the
+# group that meets the high slab begins two positions before the slab array's row.
+@pytest.mark.parametrize("dims,pml,kw", [
+    ((8, 8, 8), (1, 0, 0), {}),
+    ((40, 16, 8), (1, 1, 1), {}),
+    ((40, 16, 8), (2, 1, 3), {"arith": "fma"}),
+    ((72, 8, 16), (3, 2, 0), {"nsrc": 33}),
+    ((64, 24, 8), (5, 0, 1), {}),
+])
+def test_thin_x_slabs_equal_split(dims, pml, kw):
+    _same(_grid(dims, "auto", 11, pml, tiling=BRICK, **kw), _grid(dims, "split", 11, pml, **kw))
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16"])
+@pytest.mark.parametrize("depth", [1, 2, 3, 5])
+def test_thin_x_slabs_equal_marching_16bit(precision, depth):
+    dims, pml = (40, 16, 24), (depth, 1, 2)
+    _same(_grid(dims, "auto", 13, pml, precision=precision, tiling=BRICK),
+          _grid(dims, "fused", 13, pml, precision=precision, tiling=(4, 5, 3)))
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 5])
+def test_thin_x_slabs_around_a_marching_interior(depth):
+    dims, pml = (520, 200, 264), (depth, 9, 4)
+    _same(_grid(dims, "auto", 17, pml), _grid(dims, "split", 17, pml))
+
+
+def test_thin_x_slabs_in_a_batch():
+    sizes, depths = ((40, 16, 8), (32, 8, 8), (72, 24, 16), (8, 8, 8)), (1, 2, 3, 1)
+    dt = configs.courant_dt(1e-3)
+
+    def load(g, k):
+        nx, ny, nz = sizes[k]
+        rng = np.random.default_rng(100 + k)
+        g.set_materials(wf.MaterialGrid(wf.GridDims(nx, ny, nz)), wf.MaterialTable.vacuum_filled(dt, 1e-3))
+        for ax, n in enumerate(sizes[k]):
+            p = wf.PmlProfile1D.build(n, wf.PmlConfig(thickness=depths[k]), dt, 1e-3, depths[k])
+            g.set_pml_axis(ax, depths[k], p.b, p.a, p.inv_kappa)
+        g.set_fields(rng.standard_normal((6, nz, ny, nx)).astype(np.float32))
+        return g
+
+    b = wf.DeviceBatch([wf.GridDims(*s) for s in sizes])
+    try:
+        for k in range(len(sizes)):
+            load(b.grid(k), k)
+        b.step(6)
+        b.sync()
+        for k, s in enumerate(sizes):
+            with wf.DeviceFieldGrid(wf.GridDims(*s), kernel="split") as g:
+                load(g, k)
+                g.step(6)
+                g.sync()
+                _same([b.grid(k).fields()] + [b.grid(k).psi(w) for w in range(12)],
+                      [g.fields()] + [g.psi(w) for w in range(12)])
+    finally:
+        b.close()

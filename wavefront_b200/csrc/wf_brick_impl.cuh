@@ -133,8 +133,8 @@ __device__ __forceinline__ GroupPml group_pml(const GridArgs &g, int fl, int x, 
 }
 
 // psi index of the group's first cell on an axis (x: of its row, slab
-// position 0).  Cell and psi indices fit 32 bits here (kBrickMaxCells), so an
-// address is a uniform component base plus a 32-bit offset.
+// position 0).  Cell and psi indices stay below 2^31 here (brick_ok,
+// wf_engine.cu), so an address is a uniform component base plus a 32-bit offset.
 __device__ __forceinline__ unsigned psi_at(const GridArgs &g, const GroupPml &m, int axis, int x, int y,
                                            int z) {
   if (axis == 0) return static_cast<unsigned>((z * g.ny + y) * g.pml[0].pitch);
@@ -154,9 +154,13 @@ __device__ __forceinline__ void psi_load(const GridArgs &g, const GroupPml &m, i
     if (!idx_ok(g.err, static_cast<long long>(i) + 3, P.cells)) return;
     unpack(b_ldg4(c + i), q);
   } else {
+    // (cell 0 of a group that only ends in the slab may lie before position 0,
+    // so i + k is formed in 32 bits, where it wraps back, before the pointer)
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      q[k] = (m.xin >> k & 1u) && idx_ok(g.err, i + k, P.cells) ? __ldg(c + i + k) : 0.0f;
+    for (int k = 0; k < 4; ++k) {
+      const unsigned j = i + k;
+      q[k] = (m.xin >> k & 1u) && idx_ok(g.err, j, P.cells) ? __ldg(c + j) : 0.0f;
+    }
   }
 }
 
@@ -196,7 +200,8 @@ __device__ __forceinline__ void psi_corr(const GridArgs &g, const GroupPml &m, i
         one(v, p[k], b[k], a[k], ik[k]);
         const bool in = m.xin >> k & 1u;
         d[k] = in ? v : d[k];
-        if (store && in && idx_ok(g.err, i + k, P.cells)) o[i + k] = p[k];
+        const unsigned j = i + k;  // as in psi_load
+        if (store && in && idx_ok(g.err, j, P.cells)) o[j] = p[k];
       }
     }
   }
