@@ -344,3 +344,51 @@ def test_weight_gradient_leaves_out_taps_beyond_the_planes(n):
     assert np.isposinf(got[hit]).all()
     tol = 2.0 * (n * d * h * w + 1) ** 0.5 * 2.0 ** -24
     np.testing.assert_allclose(got[~hit], plain[~hit], rtol=tol, atol=0)
+
+
+def test_convolutions_of_several_widths_from_several_threads():
+    """Widths whose launches take different amounts of shared memory, called
+    from four threads at once, each on its own stream: every call succeeds and
+    gives the bits that it gives alone."""
+    import threading
+
+    def setup(w):
+        g = torch.Generator(device="cuda").manual_seed(w)
+        x = torch.randn(2, 16, 4, 8, w, device="cuda", generator=g)
+        wt = (0.1 * torch.randn(16, 16, 27, device="cuda", generator=g)).to(torch.bfloat16)
+        return x, wt, torch.empty_like(x)
+
+    p = lambda t: C.c_void_p(t.data_ptr())
+
+    def call(x, wt, out, stream):
+        return L.lib().wf_nn_conv3d_forward(p(x), p(wt), None, None, p(out), 2, 16, 16, 4, 8, x.shape[-1], 0,
+                                            C.c_void_p(stream.cuda_stream))
+
+    widths = (1, 12, 24, 40)
+    data = [setup(w) for w in widths]
+    streams = [torch.cuda.Stream() for _ in widths]
+    want = []
+    torch.cuda.synchronize()
+    for d, s in zip(data, streams):
+        assert call(*d, s) == 0
+        s.synchronize()
+        want.append(d[2].clone())
+    torch.cuda.synchronize()
+    bad = []
+
+    def loop(k):
+        for _ in range(2000):
+            st = call(*data[k], streams[k])
+            if st:
+                bad.append((widths[k], st))
+                return
+
+    threads = [threading.Thread(target=loop, args=(k,)) for k in range(len(widths))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not bad, bad
+    for d, w in zip(data, want):
+        assert torch.equal(d[2], w)

@@ -80,6 +80,11 @@ __host__ __device__ inline TcGeom tc_geom(int W) {
   return g;
 }
 
+// The most any width takes: the function's shared-memory limit, always the same
+// one, because it belongs to the function on the device and another thread may
+// be between its own limit and its launch with another width.
+constexpr int kTcMaxBytes = kTcWBytes + kTcZero + 16 + (kTcD + 2) * 6 * (2 * 32 + 128 + 2) * 16;
+
 __device__ unsigned long long g_tc_timeouts;  // bounded-wait expiries (diagnostic)
 
 constexpr float kInvSqrt2f = 0.70710678118654752f;
@@ -300,7 +305,8 @@ int launch_tc(const float *in, const void *w, const int *face, float *z, float *
   if (kin < 1 || kin > 16 || nout < 1 || nout > 16 || n < 1 || D < 1 || H < 1 || W < 1)
     return cudaErrorInvalidValue;
   const TcGeom G = tc_geom(W);
-  cudaError_t e = cudaFuncSetAttribute(k_conv_tc<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, G.bytes);
+  cudaError_t e =
+      cudaFuncSetAttribute(k_conv_tc<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcMaxBytes);
   if (e != cudaSuccess) return e;
   const int ndt = (D + kTcD - 1) / kTcD;
   const dim3 grid((W + G.outc - 1) / G.outc, (H + G.rows - 1) / G.rows, n * ndt);
