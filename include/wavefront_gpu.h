@@ -59,7 +59,7 @@ typedef enum {
 } wf_arith;
 
 typedef enum {
-  WF_KERNEL_AUTO = 0,  /* fused when the grid allows it, else split          */
+  WF_KERNEL_AUTO = 0,  /* the cheapest step the grid allows                  */
   WF_KERNEL_FUSED = 1, /* H and E in one pass (zero boundaries): bricks or a
                           TMA z-march                                       */
   WF_KERNEL_SPLIT = 2  /* an H kernel then an E kernel (any boundaries)      */
@@ -306,10 +306,11 @@ int64_t wf_kernel_launches(const wf_handle *h);
 
 /* {8, 4, 1} names the brick step (one CTA per 32 x 8 x 4 cells, any boundary
  * and CPML depth with FP32 storage); every other tiling is a z-march over
- * 128-cell wide tiles.  By default the cheapest for the grid's size and CPML
- * runs: either, or on large grids with x CPML the z-march over the interior
- * with bricks around it, whose tiling is then the interior's (no tiling names
- * that mix).  The results are bit-identical. */
+ * 128-cell wide tiles.  By default the cheapest for the grid's shape, CPML and
+ * boundaries runs: either, on large grids with x CPML the z-march over the
+ * interior with bricks around it, whose tiling is then the interior's, or on
+ * rows too short for bricks (kernel AUTO) the split pair; no tiling names the
+ * last two.  The results are bit-identical. */
 typedef struct {
   int32_t tile_rows;  /* y rows per CTA tile (x width is fixed at 128)      */
   int32_t z_chunk;    /* planes per CTA z-march                            */
@@ -319,8 +320,8 @@ typedef struct {
 wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out);
 wf_status wf_set_tiling(wf_handle *h, const wf_tiling *t);
 /* Times each candidate tiling for `steps` steps, and the default step where
- * it is a mix of two kernels, and keeps the fastest (`best`: as
- * wf_get_tiling reports it). */
+ * no tiling names it, and keeps the fastest (`best`: as wf_get_tiling reports
+ * it).  After wf_set_column_tiles the candidates are z-marches. */
 wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms);
 /* Fused-kernel work layout of the x-CPML slabs (no counterpart in the
  * reference, whose rayon slabs split along z only, src/engine.rs:291-422).

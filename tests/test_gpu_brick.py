@@ -186,3 +186,51 @@ def test_thin_x_slabs_in_a_batch():
                       [g.fields()] + [g.psi(w) for w in range(12)])
     finally:
         b.close()
+
+
+# The automatic step, whichever form its price picks: the split pair on short
+# rows, bricks, marching tiles.
+@pytest.mark.parametrize("dims,pml,periodic,kw", [
+    ((16, 128, 256), (4, 4, 4), "", {}),
+    ((8, 128, 256), (0, 0, 0), "xyz", {"sheet": True, "nsrc": 33}),
+    ((16, 128, 128), (4, 0, 0), "yz", {"arith": "fma"}),
+    ((24, 128, 256), (0, 0, 0), "yz", {}),
+    ((104, 264, 200), (0, 0, 0), "", {"nsrc": 33}),
+    ((136, 40, 200), (40, 3, 9), "", {}),
+])
+def test_automatic_step_equals_split(dims, pml, periodic, kw):
+    _same(_grid(dims, "auto", 19, pml, periodic, **kw), _grid(dims, "split", 19, pml, periodic, **kw))
+
+
+def test_the_form_follows_the_cpml_between_steps():
+    """A grid whose cheapest form is bricks, then the split pair, then bricks
+    again as its CPML is set: sources and probes run once a step in each."""
+    dims, steps = (16, 128, 256), 4
+    dt = configs.courant_dt(1e-3)
+    f = np.random.default_rng(23).standard_normal((6, *dims[::-1])).astype(np.float32)
+
+    def run(kernel):
+        g = wf.DeviceFieldGrid(wf.GridDims(*dims), kernel=kernel)
+        g.set_materials(wf.MaterialGrid(wf.GridDims(*dims)), wf.MaterialTable.vacuum_filled(dt, 1e-3))
+        g.set_fields(f)
+        g.add_source_values(9, 60, 100, 2, np.linspace(1.0, 2.0, 3 * steps).astype(np.float32))
+        g.add_probe_tables(8, 64, 128, 1, np.ones((3 * steps, 1)), np.full((3 * steps, 1), 2.0), 0, True)
+        out, launches = [], []
+        for t in (0, 4, 8):
+            for ax, n in enumerate(dims):
+                p = wf.PmlProfile1D.build(n, wf.PmlConfig(thickness=t), dt, 1e-3, t)
+                g.set_pml_axis(ax, t, p.b, p.a, p.inv_kappa)
+            before = g.kernel_launches
+            g.step(steps)
+            g.sync()
+            launches.append((g.kernel_launches - before) // steps)
+            out += [g.fields()] + ([g.psi(w) for w in range(12)] if t else [])
+        s = g.probe_sums(0, 1)
+        out += [s[0], s[1], np.array(s[2]), g.probe_trace(0, 3 * steps)]
+        g.close()
+        return out, launches
+
+    got, launches = run("auto")
+    want, split_launches = run("split")
+    assert launches == [1, split_launches[1], 1] and split_launches[1] > 1
+    _same(got, want)

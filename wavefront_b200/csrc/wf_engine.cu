@@ -26,6 +26,7 @@
 #include "wf_closure.h"
 #include "wf_launch.h"
 #include "wf_pool.h"
+#include "wf_price.h"
 #include "wf_scene.h"
 
 using wf::FusedArgs;
@@ -33,6 +34,7 @@ using wf::FusedConfig;
 using wf::GridArgs;
 using wf::ProbeDev;
 using wf::SrcDev;
+using wf::StepForm;
 using wf::TailArgs;
 
 namespace {
@@ -114,9 +116,8 @@ struct wf_handle {
   int test_extra_tx = 0;      // wf_set_test_stall
   bool cfg_user_set = false;  // otherwise chosen from the grid at first use
   bool col_user_set = false;  // wf_set_column_tiles was called
-  bool brick = false;         // the step runs as bricks (set with the maps)
-  bool mix = false;           // ... around an interior of marching tiles
-  int mix_lo[3] = {}, mix_hi[3] = {};
+  wf::StepForm form = wf::StepForm::kSplit;  // of the step (set with the maps)
+  wf::InteriorBox mix{};                      // kMix: the marching tiles' box
   wf::BrickMaps brick_map[2];  // per state buffer read
   wf::FusedMaps maps[2];      // per state buffer (the one read by the step)
   int *d_items = nullptr;     // work items grouped by kernel class
@@ -365,90 +366,31 @@ bool is_brick(const FusedConfig &c) {
   return c.ty == wf::kBrickY && c.zchunk == wf::kBrickZ && c.stages == 1;
 }
 
-// Where an automatic step on CPML runs both: the marching tiles' interior
-// class over the cells whose step, halo and warm-up plane meet no slab, cut to
-// whole bricks, and bricks around it.  False where either cannot run or there
-// is no such box.
-struct MixBox {
-  int lo[3], hi[3];
-};
-bool mix_box(const wf_handle *h, MixBox *m) {
-  if (!brick_ok(h) || !marching_ok(h)) return false;
-  const int brick[3] = {wf::kBrickX, wf::kBrickY, wf::kBrickZ};
-  bool pml = false;
+static_assert(wf::price::kBrick[0] == wf::kBrickX && wf::price::kBrick[1] == wf::kBrickY &&
+                  wf::price::kBrick[2] == wf::kBrickZ && wf::price::kTileWide == wf::kTileX &&
+                  wf::price::kColumnWide == wf::kColWidth && wf::price::kColumnRows == wf::kColTileRows,
+              "the prices count what the kernels launch");
+
+wf::StepShape step_shape(const wf_handle *h) {
+  wf::StepShape s{{h->nx, h->ny, h->nz}, {}, {}, store16(h)};
   for (int a = 0; a < 3; ++a) {
-    const int n = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz), T = h->ax[a].T, b = brick[a];
-    pml = pml || T > 0;
-    m->lo[a] = T > 0 ? T / b * b + b : 0;
-    m->hi[a] = T > 0 ? (n - T) / b * b : n;
-    if (m->hi[a] <= m->lo[a]) return false;
+    s.depth[a] = h->ax[a].T;
+    s.periodic[a] = h->periodic[a] != 0;
   }
-  return pml;
+  return s;
 }
 
-// CPML cells of the grid, in millions.
-double shell_cells(const wf_handle *h) {
-  const double n = 1e-6 * static_cast<double>(h->N);
-  double inner = n;
-  for (int a = 0; a < 3; ++a) {
-    const int len = a == 0 ? h->nx : (a == 1 ? h->ny : h->nz);
-    inner *= static_cast<double>(len - h->ax[a].W) / len;
-  }
-  return n - inner;
+// The form of the handle's step: a tiling or column-tile choice of the
+// caller's decides between bricks and marching tiles (where those cannot run,
+// the split pair), otherwise the cheapest by price (wf_price.h).  kernel=fused
+// takes the split pair only where nothing else can run.
+StepForm step_form(const wf_handle *h) {
+  const bool march = marching_ok(h), brick = brick_ok(h);
+  if (h->cfg_user_set && brick && is_brick(h->cfg)) return StepForm::kBrick;
+  if (h->cfg_user_set || h->col_user_set || !(march || brick))
+    return march ? StepForm::kMarch : StepForm::kSplit;
+  return wf::cheapest_step(step_shape(h), march, brick, h->kernel_pref == WF_KERNEL_AUTO);
 }
-
-// Interior cells run at 8.4 to 8.9 us per million as marching tiles and 12.6
-// as bricks of the CPML kernel; the shell at 18 to 20 as bricks, while the
-// marching tiles pay most for the x slabs (36 per million cells of their
-// columns; with y and z slabs only there is nothing to gain).  The cheapest
-// by their times on B200, per million cells n, CPML cells s and interior
-// cells i (two launches, a join and a separate tail: 40):
-//   FP32    bricks 12.6 n + 6.9 s, marching 8 n + 22 s + 100,
-//           both 8.4 i + 18.4 (n - i) + 40 (22 where slabs are not aligned)
-//   16-bit  13.9 n, 6.5 n + 22 s + 100, 6.9 i + 19 (n - i) + 40
-// 16 CPML cells: FP32 320^3 464 -> 437 us, 384^3 792 -> 736, 512^3 1735 ->
-// 1583, 1024^3 10448 -> 10292; binary16 320^3 457 -> 382, 512^3 1605 -> 1373.
-// Eight cells, vacuum: 384^3 750 -> 649, 512^3 1394 and 1400, 768^3 4155
-// marching and 4361 both, so marching.
-bool use_mix(const wf_handle *h, MixBox *m) {
-  if (h->cfg_user_set || h->col_user_set || h->ax[0].T == 0 || !mix_box(h, m)) return false;
-  const double n = 1e-6 * static_cast<double>(h->N), s = shell_cells(h);
-  const double i = 1e-6 * (m->hi[0] - m->lo[0]) * static_cast<double>(m->hi[1] - m->lo[1]) *
-                   (m->hi[2] - m->lo[2]);
-  const bool b16 = store16(h);
-  const double bricks = b16 ? 13.9 * n : 12.6 * n + 6.9 * s;
-  const double marching = (b16 ? 6.5 : 8.0) * n + 22.0 * s + 100.0;
-  const double outer = b16 ? 19.0 : (h->ax[0].T % 4 ? 22.0 : 18.4);
-  return (b16 ? 6.9 : 8.4) * i + outer * (n - i) + 40.0 < std::min(bricks, marching);
-}
-
-// Whether the step runs as bricks rather than as marching tiles (or, where
-// neither can, as the split pair).  Unless the caller chose a tiling or the
-// column tiles, the cheaper of the two by their times on B200, in
-// microseconds per million cells (cubes of 64 to 640 cells, 0- to 16-cell
-// CPML):
-//   FP32, marching  N / 120e3 + 23 us per million CPML cells + 100 us for the
-//                   chain of its slowest class (none without CPML);
-//   FP32, bricks    N / 95e3 + 19 us per million CPML cells
-//                   (256^3, 8-cell CPML: 298 -> 233 us; 64^3: 51.9 -> 6.8;
-//                   512^3, 16-cell: 1747 and 1850, so marching; 512^3 without
-//                   CPML: 1119 and 1364, marching);
-//   16-bit          375 us + 9.2 us per million cells marching against 13.5
-//                   us bricks (320^3: 676 -> 478; 512^3: 1606 and 1812).
-bool use_brick(const wf_handle *h) {
-  if (!brick_ok(h)) return false;
-  if (h->cfg_user_set) return is_brick(h->cfg);
-  if (h->col_user_set) return false;
-  if (!marching_ok(h)) return true;
-  MixBox m;
-  if (use_mix(h, &m)) return true;
-  const double n = 1e-6 * static_cast<double>(h->N);
-  if (store16(h)) return n < 86.0;
-  const double shell = shell_cells(h);
-  return 2.2 * n < (shell > 0.0 ? 100.0 + 4.0 * shell : 4.0);
-}
-
-bool use_fused(const wf_handle *h) { return use_brick(h) || marching_ok(h); }
 
 bool has_pml(const wf_handle *h) { return h->ax[0].T > 0 || h->ax[1].T > 0 || h->ax[2].T > 0; }
 FusedArgs fused_args(const wf_handle *h);
@@ -502,20 +444,13 @@ void brick_geometry(BrickGrid *a) {
 namespace {
 
 // Tiling used unless the caller set one: 4 rows, 3 stages, and the z chunk
-// measured best on B200 (two_spheres 512^3, random spheres 1024^3).  A
-// longer chunk recomputes the warm-up plane less often; the issue-bound
-// 16-bit kernel gains most from that.
+// measured best on B200 (two_spheres 512^3, random spheres 1024^3).
 FusedConfig default_cfg(const wf_handle *h) {
-  MixBox m{{0, 0, 0}, {h->nx, h->ny, h->nz}};
-  if (!use_mix(h, &m)) m = MixBox{{0, 0, 0}, {h->nx, h->ny, h->nz}};
-  const int nx = m.hi[0] - m.lo[0], ny = m.hi[1] - m.lo[1], nz = m.hi[2] - m.lo[2];
-  const bool big = h->nz >= 1024;
-  if (store16(h)) return FusedConfig{4, big ? 48 : 32, 3};
-  // FP32: 24-plane chunks (fewer warm-up planes) while they still give at
-  // least four waves of work items at three CTAs per SM, else 12
-  const long long tiles = static_cast<long long>((nx + wf::kTileX - 1) / wf::kTileX) * ((ny + 3) / 4);
-  const long long items24 = tiles * ((nz + 23) / 24);
-  return FusedConfig{4, items24 >= 4LL * 148 * 3 ? 24 : 12, 3};
+  wf::InteriorBox b{};
+  if (!(step_form(h) == StepForm::kMix && wf::interior_box(step_shape(h), &b)))
+    b = wf::InteriorBox{{0, 0, 0}, {h->nx, h->ny, h->nz}};
+  const int m[3] = {b.hi[0] - b.lo[0], b.hi[1] - b.lo[1], b.hi[2] - b.lo[2]};
+  return FusedConfig{4, wf::price::march_chunk(m, h->nz, store16(h)), 3};
 }
 
 // TMA descriptors per state buffer: fields as a 4D tensor {nx, ny, nz, 6},
@@ -523,6 +458,12 @@ FusedConfig default_cfg(const wf_handle *h) {
 // axis's psi slab as a 4D tensor {.., .., .., 4 terms}.
 wf_status build_maps(wf_handle *h, bool allow_cols = true) {
   h->maps_ok = false;
+  h->form = step_form(h);
+  if (h->form == StepForm::kSplit) {  // the pair needs no descriptors
+    h->cols = false;
+    h->maps_ok = true;
+    return WF_OK;
+  }
   if (!encode_fn()) return fail(h, WF_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
   if (!h->cfg_user_set) h->cfg = default_cfg(h);
   h->cols = allow_cols && cols_apply(h);
@@ -537,18 +478,14 @@ wf_status build_maps(wf_handle *h, bool allow_cols = true) {
                                                                 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   const cuuint64_t mdim[3] = {(cuuint64_t)h->nx, (cuuint64_t)h->ny, (cuuint64_t)h->nz};
   const cuuint64_t mstr[2] = {(cuuint64_t)h->mat_pitch, (cuuint64_t)h->mat_pitch * h->ny};
-  h->brick = use_brick(h);
-  MixBox mix{};
-  h->mix = h->brick && use_mix(h, &mix);
-  std::copy(std::begin(mix.lo), std::end(mix.lo), h->mix_lo);
-  std::copy(std::begin(mix.hi), std::end(mix.hi), h->mix_hi);
-  if (h->brick) {
+  if (h->form == StepForm::kMix) wf::interior_box(step_shape(h), &h->mix);
+  if (h->form != StepForm::kMarch) {
     h->cols = false;
     for (int b = 0; b < 2; ++b)
       if (!wf::brick_encode(&h->brick_map[b], h->fld[b], h->nx, h->ny, h->nz, h->precision))
         return fail(h, WF_ERR_CUDA, "cuTensorMapEncodeTiled(bricks) failed");
     WF_CUDA(h, wf::brick_prepare(h->precision, h->arith == WF_ARITH_FMA));
-    if (!h->mix) {
+    if (h->form == StepForm::kBrick) {
       h->maps_ok = true;
       return WF_OK;
     }
@@ -590,7 +527,7 @@ wf_status build_maps(wf_handle *h, bool allow_cols = true) {
   for (int k = 0; k < wf::kFusedClassCount; ++k) {
     h->class_off[k] = static_cast<int>(all.size());
     h->class_n[k] = static_cast<int>(lists[k].size());
-    if (h->mix && k > 0 && h->class_n[k]) return fail(h, WF_ERR_CUDA, "an interior item meets a CPML slab");
+    if (h->form == StepForm::kMix && k > 0 && h->class_n[k]) return fail(h, WF_ERR_CUDA, "an interior item meets a CPML slab");
     all.insert(all.end(), lists[k].begin(), lists[k].end());
   }
   // column items (low and high x edge, 32-row tiles), one list per class
@@ -759,13 +696,14 @@ TailArgs tail_args(const wf_handle *h) {
 FusedArgs fused_args(const wf_handle *h) {
   FusedArgs a{};
   a.g = grid_args(h);
-  a.x_lo = h->mix ? h->mix_lo[0] : (h->cols ? wf::kColWidth : 0);
-  a.x_hi = h->mix ? h->mix_hi[0] : (h->cols ? h->nx - wf::kColWidth : h->nx);
-  a.y_lo = h->mix ? h->mix_lo[1] : 0;
-  a.z_lo = h->mix ? h->mix_lo[2] : 0;
-  a.z_hi = h->mix ? h->mix_hi[2] : h->nz;
+  const bool mix = h->form == StepForm::kMix;
+  a.x_lo = mix ? h->mix.lo[0] : (h->cols ? wf::kColWidth : 0);
+  a.x_hi = mix ? h->mix.hi[0] : (h->cols ? h->nx - wf::kColWidth : h->nx);
+  a.y_lo = mix ? h->mix.lo[1] : 0;
+  a.z_lo = mix ? h->mix.lo[2] : 0;
+  a.z_hi = mix ? h->mix.hi[2] : h->nz;
   a.tiles_x = (a.x_hi - a.x_lo + wf::kTileX - 1) / wf::kTileX;
-  a.tiles_y = ((h->mix ? h->mix_hi[1] - h->mix_lo[1] : h->ny) + h->cfg.ty - 1) / h->cfg.ty;
+  a.tiles_y = ((mix ? h->mix.hi[1] - h->mix.lo[1] : h->ny) + h->cfg.ty - 1) / h->cfg.ty;
   a.zchunk = h->cfg.zchunk;
   a.has_pml = has_pml(h) ? 1 : 0;
   a.prof_in_smem = (h->ax[0].W <= 64 && h->ax[1].W <= 64 && h->ax[2].W <= 64) ? 1 : 0;
@@ -795,7 +733,7 @@ cudaEvent_t timing_event(wf_handle *h) {
 // Whether a brick step applies the sources and probes itself: few of them,
 // and nothing (the closure) between the step and its sources.
 bool brick_tail(const wf_handle *h) {
-  return h->brick && !h->mix && !store16(h) && !h->closure && (!h->srcs.empty() || !h->probes.empty()) &&
+  return h->form == StepForm::kBrick && !store16(h) && !h->closure && (!h->srcs.empty() || !h->probes.empty()) &&
          h->srcs.size() <= wf::kBrickTailMax && h->probes.size() <= wf::kBrickTailMax;
 }
 
@@ -805,8 +743,8 @@ wf::BrickShell mix_shell(const wf_handle *h) {
   int lo[3], hi[3], all[3];
   for (int a = 0; a < 3; ++a) {
     all[a] = (n[a] + b[a] - 1) / b[a];
-    lo[a] = h->mix_lo[a] / b[a];
-    hi[a] = (h->mix_hi[a] + b[a] - 1) / b[a];
+    lo[a] = h->mix.lo[a] / b[a];
+    hi[a] = (h->mix.hi[a] + b[a] - 1) / b[a];
   }
   wf::BrickShell s{};
   int box = 0;
@@ -839,8 +777,18 @@ wf::BrickArgs brick_args(const wf_handle *h) {
     a.tail.step = h->d_step + h->cur;
     a.tail.step_next = h->d_step + (h->cur ^ 1);
   }
-  if (h->mix) a.shell = mix_shell(h);
+  if (h->form == StepForm::kMix) a.shell = mix_shell(h);
   return a;
+}
+
+// What the handle's step needs before its first launch.
+wf_status ready_step(wf_handle *h) {
+  if (!h->maps_ok) {
+    const wf_status s = build_maps(h);
+    if (s != WF_OK) return s;
+  }
+  if ((h->form == StepForm::kMarch || h->form == StepForm::kMix) && !h->fork_ev) return acquire_streams(h);
+  return WF_OK;
 }
 
 wf_status enqueue_one(wf_handle *h) {
@@ -856,17 +804,8 @@ wf_status enqueue_one(wf_handle *h) {
     if (!ev) return fail(h, WF_ERR_CUDA, "cudaEventCreate");
     WF_CUDA(h, cudaEventRecord(ev, h->stream));
   }
-  if (use_fused(h)) {
-    if (!h->maps_ok) {
-      wf_status s = build_maps(h);
-      if (s != WF_OK) return s;
-    }
-    if ((!h->brick || h->mix) && !h->fork_ev) {
-      wf_status s = acquire_streams(h);
-      if (s != WF_OK) return s;
-    }
-  }
-  if (use_fused(h) && h->mix) {
+  if (wf_status s = ready_step(h); s != WF_OK) return s;
+  if (h->form == StepForm::kMix) {
     // the interior on a side stream, first: its items are the long ones, and
     // the bricks fill the SMs as they end; disjoint cells of the next state
     WF_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
@@ -879,10 +818,10 @@ wf_status enqueue_one(wf_handle *h) {
       WF_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[0], 0));
     }
     if (e == cudaSuccess) h->kernel_launches += 2;
-  } else if (use_fused(h) && h->brick) {
+  } else if (h->form == StepForm::kBrick) {
     e = wf::launch_brick(h->brick_map[h->cur], brick_args(h), fma, h->stream);
     if (e == cudaSuccess) h->kernel_launches += 1;
-  } else if (use_fused(h)) {
+  } else if (h->form == StepForm::kMarch) {
     const FusedArgs a = fused_args(h);
     // class 0 (interior) on the main stream, the CPML classes on side
     // streams forked from it; they touch disjoint cells of the next state.
@@ -1111,7 +1050,8 @@ wf_status narrow_batch_maps(wf_handle *h, int zchunk, wf::BatchScene *sc) {
   const int cur = h->cur;
   const FusedConfig saved = h->cfg;
   h->cfg = FusedConfig{wf::kColTileRows, zchunk, 3};
-  h->cols = h->mix = false;
+  h->cols = false;
+  h->form = StepForm::kMarch;  // fused_args below: the whole grid
   for (int p = 0; p < 2; ++p) {
     CUtensorMap *m = sc->maps[p];
     std::memset(m, 0, sizeof(CUtensorMap) * 3);
@@ -1770,17 +1710,11 @@ wf_status wf_step(wf_handle *h, int nsteps) {
   std::string why;
   if (!tables_cover(h, h->steps_done + nsteps, &why)) return fail(h, WF_ERR_ARG, why);
   DeviceGuard guard(h->dev);
-  if (store16(h) && !use_fused(h))
+  if (store16(h) && !marching_ok(h))
     return fail(h, WF_ERR_UNSUPPORTED,
                 "16-bit storage runs the fused kernel only: CPML slabs of at most 64 cells");
-  if (use_fused(h) && !h->maps_ok) {  // descriptors + smem limit, outside any capture
-    wf_status s = build_maps(h);
-    if (s != WF_OK) return s;
-  }
-  if (use_fused(h) && (!h->brick || h->mix) && !h->fork_ev) {  // the side streams, outside any capture too
-    wf_status s = acquire_streams(h);
-    if (s != WF_OK) return s;
-  }
+  // descriptors, shared-memory limits and side streams, outside any capture
+  if (wf_status s = ready_step(h); s != WF_OK) return s;
   if (h->tables_dirty) {  // sources/probes added since the last step
     wf_status s = flush_tables(h);
     if (s != WF_OK) return s;
@@ -2123,10 +2057,10 @@ wf_status wf_set_test_stall(wf_handle *h, int extra_bytes) {
 
 wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out) {
   if (!h || !out) return WF_ERR_ARG;
-  MixBox m;  // a mixed step reports its interior's tiling
-  const FusedConfig c = h->cfg_user_set ? h->cfg
-                        : use_brick(h) && !use_mix(h, &m) ? FusedConfig{wf::kBrickY, wf::kBrickZ, 1}
-                                        : default_cfg(h);
+  // a mixed step reports its interior's tiling
+  const FusedConfig c = h->cfg_user_set                     ? h->cfg
+                        : step_form(h) == StepForm::kBrick ? FusedConfig{wf::kBrickY, wf::kBrickZ, 1}
+                                                           : default_cfg(h);
   out->tile_rows = c.ty;
   out->z_chunk = c.zchunk;
   out->stages = c.stages;
@@ -2162,7 +2096,7 @@ wf_status wf_set_column_tiles(wf_handle *h, int enable) {
 
 int wf_column_tiles_active(const wf_handle *h) {
   if (!h) return -1;
-  if (!use_fused(h) || use_brick(h)) return 0;
+  if ((h->maps_ok ? h->form : step_form(h)) != StepForm::kMarch) return 0;
   return (h->maps_ok ? h->cols : cols_apply(h)) ? 1 : 0;
 }
 
@@ -2179,11 +2113,13 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   const FusedConfig orig = h->cfg;
   const int orig_cur = h->cur;
   std::vector<FusedConfig> cands;
-  // the automatic step first where it mixes bricks and marching tiles (0 rows
-  // here: no tiling names it); every other trial is an explicit tiling
-  MixBox m;
-  if (use_mix(h, &m)) cands.push_back(FusedConfig{0, 0, 0});
-  if (brick_ok(h)) cands.push_back(FusedConfig{wf::kBrickY, wf::kBrickZ, 1});
+  // the automatic step first where no tiling names it (0 rows here): a mix of
+  // bricks and marching tiles, or the split pair; every other trial is an
+  // explicit tiling
+  h->cfg_user_set = false;
+  const StepForm automatic = step_form(h);
+  if (automatic == StepForm::kMix || automatic == StepForm::kSplit) cands.push_back(FusedConfig{0, 0, 0});
+  if (brick_ok(h) && !h->col_user_set) cands.push_back(FusedConfig{wf::kBrickY, wf::kBrickZ, 1});
   const int tys[] = {4, 8, 16};
   const int stg[] = {3, 4};
   const int zcs[] = {16, 32, 64, 128, 1 << 20};

@@ -8,7 +8,8 @@
 // without allocating anything.
 //
 // It runs the brick step (wf_brick_impl.cuh; the split H and E kernels of
-// wf_split.cu where the buffers' alignment rules bricks out) with the caller's
+// wf_split.cu where the buffers' alignment rules bricks out or rows are too
+// short for them) with the caller's
 // fields as one state buffer and a file-scope static device array as the other
 // (the next-state buffer the kernels write).  The array has a fixed maximum
 // size; every GPU that loads this library holds it until the process exits.
@@ -17,6 +18,7 @@
 
 #include "../../include/wavefront_gpu.h"
 #include "wf_launch.h"
+#include "wf_price.h"
 
 namespace {
 
@@ -174,9 +176,13 @@ wf_status wf_step_fields_noalloc(float *fields6, const uint8_t *ids,
   g.err = nullptr;  // no error word: a brick whose copy never lands writes NaN
   float *bufs[2] = {fields6, sc->next_state};
   // One brick launch per step where the caller's buffers allow its 16-byte
-  // boxes and 4-byte id loads (64^3: 12.5 -> 5 us a step), else the split pair.
+  // boxes and 4-byte id loads (64^3: 12.4 -> 5.1 us a step) and rows are not so
+  // short that the split pair is cheaper (8 x 128 x 256: 12.4 against 15.2).
   wf::BrickMaps maps[2];
-  bool brick = reinterpret_cast<uintptr_t>(fields6) % 16 == 0 && reinterpret_cast<uintptr_t>(ids) % 4 == 0;
+  wf::StepShape shape{{nx, ny, nz}, {}, {}, false};
+  for (int i = 0; i < 3; ++i) shape.periodic[i] = g.periodic[i] != 0;
+  bool brick = wf::price::brick_us(shape) <= wf::price::split_us(shape) &&
+               reinterpret_cast<uintptr_t>(fields6) % 16 == 0 && reinterpret_cast<uintptr_t>(ids) % 4 == 0;
   for (int b = 0; b < 2 && brick && nsteps > 0; ++b)
     brick = wf::brick_encode(&maps[b], bufs[b], nx, ny, nz, wf::kPrecF32);
   if (brick && nsteps > 0) {
