@@ -107,3 +107,43 @@ def test_batch_requires_lockstep():
             b.step(1)
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("tiling", [(4, 16, 3), (32, 16, 3), (8, 4, 1)])
+def test_grids_stepped_alone_around_batched_steps(tiling):
+    """Each grid alone for 40 steps (a captured graph of 32 among them), the
+    batch for 33, each alone again: building the batch replaces a grid's
+    descriptors and work lists, so the graph captured before must not be
+    replayed after."""
+    sizes = (64, 48)
+    scenes = configs.batched_sweep(2, steps=113, seed=29, sizes=(64,))[:1] + configs.batched_sweep(
+        1, steps=113, seed=31, sizes=(48,))
+    b = configs.device_batch(scenes)
+    try:
+        b.set_tiling(*tiling)
+        for g in b.grids:
+            g.set_tiling(4, 12, 3)
+        for g in b.grids:
+            g.step(40)
+        b.step(33)
+        for g in b.grids:
+            g.step(40)
+        b.sync()
+        for i, sc in enumerate(scenes):
+            assert sc.dims.nx == sizes[i]
+            h = configs.device_grid(sc, kernel="split")
+            for s_ in sc.sources:
+                h.add_source_values(s_.x, s_.y, s_.z, s_.component, s_.values(sc.dt, 113), s_.mode)
+            for p_ in sc.probes:
+                c, si = p_.tables(sc.dt, 113)
+                h.add_probe_tables(p_.x, p_.y, p_.z, p_.component, c, si, p_.first_step(sc.dt))
+            h.step(113)
+            h.sync()
+            _eq(b.grid(i).fields(), h.fields(), f"grid {i} fields")
+            for w in range(12):
+                _eq(b.grid(i).psi(w), h.psi(w), f"grid {i} {wf.PSI_NAMES[w]}")
+            a, z = b.grid(i).probe_sums(0, 1), h.probe_sums(0, 1)
+            assert np.array_equal(a[0], z[0]) and np.array_equal(a[1], z[1]) and a[2] == z[2]
+            h.close()
+    finally:
+        b.close()

@@ -458,6 +458,7 @@ FusedConfig default_cfg(const wf_handle *h) {
 // axis's psi slab as a 4D tensor {.., .., .., 4 terms}.
 wf_status build_maps(wf_handle *h, bool allow_cols = true) {
   h->maps_ok = false;
+  drop_graphs(h);  // captured steps hold the old descriptors and work lists
   h->form = step_form(h);
   if (h->form == StepForm::kSplit) {  // the pair needs no descriptors
     h->cols = false;
