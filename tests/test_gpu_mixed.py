@@ -196,3 +196,31 @@ def test_mixed_precision_error_vs_fp64(oracle):
         assert ov == 0, prec
         assert max(fe) < fb, (prec, fe)
         assert a < pb, (prec, a)
+
+
+@pytest.mark.parametrize("precision", ["f16", "bf16", "f32"])
+def test_autotune_keeps_sources_and_probes(precision):
+    """Sources and probes added before the autotuner runs act in the steps
+    after it: equal to a grid that was never tuned, bit for bit."""
+    sc = configs.two_spheres(n=64, steps=24)
+
+    def run(tune):
+        g = configs.device_grid(sc, precision=precision)
+        for s in sc.sources:
+            g.add_source_values(s.x, s.y, s.z, s.component, s.values(sc.dt, 24), s.mode)
+        for p in sc.probes:
+            c, si = p.tables(sc.dt, 24)
+            g.add_probe_tables(p.x, p.y, p.z, p.component, c, si, p.first_step(sc.dt))
+        if tune:
+            g.autotune(2)
+        g.step(24)
+        g.sync()
+        out = [g.fields()] + [v for i, p in enumerate(sc.probes)
+                              for v in map(np.asarray, g.probe_sums(i, len(p.frequencies_hz)))]
+        g.close()
+        return out
+
+    want, got = run(False), run(True)
+    assert np.abs(want[0]).max() > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)

@@ -2136,6 +2136,9 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms) 
   float bms = 1e30f;
   FusedConfig bc = orig;
   // Source/probe tails are excluded: tuning times the stencil alone.
+  // The trials run without sources and probes.  Their descriptors go up first:
+  // a 16-bit trial's tail would take the empty lists for the grid's.
+  if ((st = flush_tables(h)) != WF_OK) return st;
   std::vector<SrcRec> srcs;
   std::vector<ProbeRec> probes;
   srcs.swap(h->srcs);
