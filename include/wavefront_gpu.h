@@ -432,10 +432,11 @@ wf_status wf_batch_get_tiling(const wf_batch *b, wf_tiling *out);
 wf_status wf_batch_set_tiling(wf_batch *b, const wf_tiling *t);
 /* Times the batched step kernel for `steps` steps under each instantiated
  * tiling and z chunk, keeps the fastest, and restores every grid's fields
- * and psi (sources and probes do not run during the trials).  The brick step,
- * a new batch's default, is timed too and stays in use (wf_batch_get_tiling
- * {8, 4, 1}) when no z-march beats it; best and best_ms always describe the
- * fastest z-march. */
+ * and psi (sources and probes do not run during the trials).  The brick step
+ * is timed too and stays in use (wf_batch_get_tiling {8, 4, 1}) when no
+ * z-march beats it; best and best_ms always describe the fastest z-march.
+ * A batch that was neither tuned nor given a tiling takes the cheaper of
+ * bricks and 4-row, 16-plane marching items by its grids' shapes and CPML. */
 wf_status wf_batch_autotune(wf_batch *b, int steps, wf_tiling *best, float *best_ms);
 
 /* ---- device memory cache (no reference counterpart) ---------------------- */

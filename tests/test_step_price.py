@@ -105,3 +105,39 @@ def test_marching_and_bricks_stay_within_what_can_run(pick):
     # nothing marches on periodic axes or over slabs of more than 64 positions
     got = pick([(512, 512, 512, 0, 0, 0, 0, 1, 1, 0, 0), (256, 256, 256, 40, 40, 40, 0, 0, 0, 0, 0)])
     assert all(f in ("split", "brick") for f in got)
+
+
+# (grids, cells of an edge, CPML depth, us as bricks, us as marching items)
+BATCHES = [
+    (4, 256, 0, 932.3, 576.9), (4, 256, 10, 1115.3, 1379.9), (4, 256, 8, 1017.0, 939.5), (3, 320, 16, 1534.5, 1629.4),
+    (16, 128, 0, 460.2, 302.3), (16, 128, 10, 641.1, 974.1), (20, 104, 0, 381.5, 223.8), (48, 40, 0, 85.8, 91.8),
+    (48, 40, 4, 115.0, 215.8), (32, 72, 0, 225.3, 163.9), (32, 72, 8, 296.0, 401.6), (3, 64, 10, 24.6, 100.3),
+    (3, 32, 0, 6.8, 25.2), (60, 96, 0, 734.4, 527.6), (60, 96, 8, 961.2, 1194.2), (1, 512, 8, 1927.8, 1568.5),
+    (1, 448, 0, 1252.9, 844.2), (60, 24, 4, 37.7, 132.2),
+]
+
+BATCH_MAIN = r'''
+#include "wf_price.h"
+#include <cstdio>
+#include <vector>
+int main() {
+  int n, e, t;
+  while (scanf("%d%d%d", &n, &e, &t) == 3) {
+    const std::vector<wf::StepShape> v(n, wf::StepShape{{e, e, e}, {t, t, t}, {}, false});
+    printf("%d\n", wf::batch_takes_bricks(v.data(), n) ? 1 : 0);
+  }
+}
+'''
+
+
+def test_a_batch_takes_the_faster_measured_form(tmp_path):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no host compiler")
+    (tmp_path / "batch.cpp").write_text(BATCH_MAIN)
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", CSRC, str(tmp_path / "batch.cpp"), "-o", str(tmp_path / "batch")],
+                   check=True)
+    lines = "".join(f"{n} {e} {t}\n" for n, e, t, _, _ in BATCHES)
+    out = subprocess.run([str(tmp_path / "batch")], input=lines, capture_output=True, text=True, check=True).stdout
+    for (n, e, t, bricks, march), v in zip(BATCHES, out.split()):
+        assert (bricks if v == "1" else march) <= 1.08 * min(bricks, march), (n, e, t, v)

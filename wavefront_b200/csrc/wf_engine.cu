@@ -978,15 +978,16 @@ wf_status check_device_error(wf_handle *h) {
 }  // namespace
 
 // A batch of independent grids stepped by one launch per step
-// (many small scenes of uneven size): the bricks of every grid, or with a
-// z-march tiling set one persistent launch per CPML class.  Each grid is an ordinary
+// (many small scenes of uneven size): the bricks of every grid, or one
+// persistent launch of marching items per CPML class.  Each grid is an ordinary
 // handle on the batch's stream; the batch keeps device tables describing
 // all of them for the batched step kernel and the batched tail.
 struct wf_batch {
   int dev = 0;
   cudaStream_t stream = nullptr;
   std::vector<wf_handle *> h;
-  FusedConfig cfg{wf::kBrickY, wf::kBrickZ, 1};  // bricks unless a tiling is set
+  FusedConfig cfg{4, wf::price::kBatchChunk, 3};  // of the tables (batch_cfg)
+  bool cfg_user_set = false;
   wf::BatchScene *d_scenes = nullptr;
   // brick form: the grids' maps and arguments, one item per brick
   wf::BrickScene *d_bricks = nullptr;
@@ -1091,6 +1092,17 @@ int narrow_item_class(const FusedArgs &a, int k) {
 }
 
 // (Re)builds the batch's device tables when any grid's tables changed.
+// The tiling a batch runs: the caller's, or the cheaper of bricks and marching
+// items (wf_price.h).
+FusedConfig batch_cfg(const wf_batch *b) {
+  if (b->cfg_user_set) return b->cfg;
+  std::vector<wf::StepShape> shapes;
+  for (const wf_handle *h : b->h) shapes.push_back(step_shape(h));
+  if (wf::batch_takes_bricks(shapes.data(), static_cast<int>(shapes.size())))
+    return FusedConfig{wf::kBrickY, wf::kBrickZ, 1};
+  return FusedConfig{4, wf::price::kBatchChunk, 3};
+}
+
 wf_status batch_build(wf_batch *b) {
   bool fresh = b->built && b->versions.size() == b->h.size();
   for (size_t i = 0; fresh && i < b->h.size(); ++i) fresh = b->versions[i] == b->h[i]->version;
@@ -1101,6 +1113,7 @@ wf_status batch_build(wf_batch *b) {
   std::vector<int2> lists[wf::kFusedClassCount];
   std::vector<TailArgs> tails[2];
   b->have_tail = false;
+  b->cfg = batch_cfg(b);
   b->narrow = wf::fused_batch_narrow(b->cfg);
   b->brick = is_brick(b->cfg);
   b->brick_xs = false;
@@ -1111,6 +1124,8 @@ wf_status batch_build(wf_batch *b) {
       if (A.T > 0 && A.W > 64)
         return fail(nullptr, WF_ERR_UNSUPPORTED, "batched grids need CPML slabs of at most 64 cells");
     wf_status st = WF_OK;
+    const FusedConfig own = h->cfg;
+    const bool own_set = h->cfg_user_set;
     if (b->brick) {
       if (!brick_ok(h)) return fail(nullptr, WF_ERR_UNSUPPORTED, "a batched grid is too large for bricks");
       for (int p = 0; p < 2; ++p)
@@ -1120,12 +1135,19 @@ wf_status batch_build(wf_batch *b) {
     } else if (b->narrow) {
       st = narrow_batch_maps(h, b->cfg.zchunk, &scenes[i]);
     } else {
+      // the batch's tiling for this build; a step of the grid alone keeps its own
+      // and rebuilds its descriptors
       h->cfg = b->cfg;
       h->cfg_user_set = true;
       st = build_maps(h, false);  // the batched kernel tiles the whole x range
+      h->maps_ok = false;
     }
     if (st == WF_OK) st = flush_tables(h);
-    if (st != WF_OK) return st;
+    if (st != WF_OK) {
+      h->cfg = own;
+      h->cfg_user_set = own_set;
+      return st;
+    }
     const int cur = h->cur;
     for (int p = 0; p < 2; ++p) {
       h->cur = p;
@@ -1144,6 +1166,8 @@ wf_status batch_build(wf_batch *b) {
       tails[p].push_back(tail_args(h));
     }
     h->cur = cur;
+    h->cfg = own;
+    h->cfg_user_set = own_set;
     if (!h->srcs.empty() || !h->probes.empty()) b->have_tail = true;
     if (b->brick) continue;
     const FusedArgs &a = scenes[i].args[0];
@@ -2805,14 +2829,16 @@ wf_status wf_batch_set_tiling(wf_batch *b, const wf_tiling *t) {
   WF_CUDA(nullptr, cudaStreamSynchronize(b->stream));
   batch_drop(b);
   b->cfg = c;
+  b->cfg_user_set = true;
   return WF_OK;
 }
 
 wf_status wf_batch_get_tiling(const wf_batch *b, wf_tiling *out) {
   if (!b || !out) return fail(nullptr, WF_ERR_ARG, "null argument");
-  out->tile_rows = b->cfg.ty;
-  out->z_chunk = b->cfg.zchunk;
-  out->stages = b->cfg.stages;
+  const FusedConfig c = batch_cfg(b);
+  out->tile_rows = c.ty;
+  out->z_chunk = c.zchunk;
+  out->stages = c.stages;
   return WF_OK;
 }
 
@@ -2923,6 +2949,7 @@ wf_status wf_batch_autotune(wf_batch *b, int steps, wf_tiling *best, float *best
   auto trial = [&](const FusedConfig &c) {  // milliseconds a step, or < 0
     batch_drop(b);
     b->cfg = c;
+    b->cfg_user_set = true;
     if (batch_build(b) != WF_OK) return -1.0f;
     int parity = cur0;
     bool okc = batch_kernel(b, parity) == WF_OK;  // warm-up
