@@ -234,3 +234,44 @@ def test_the_form_follows_the_cpml_between_steps():
     want, split_launches = run("split")
     assert launches == [1, split_launches[1], 1] and split_launches[1] > 1
     _same(got, want)
+
+
+def test_grids_beyond_a_brick_launch_run_other_forms():
+    """More than 65535 bands of 64 rows do not fit a launch of bricks: the tiling
+    is refused, a step and a batch of such a grid (13 GB) run other forms."""
+    dims, steps = wf.GridDims(8, 4194312, 8), 3
+
+    def load(g):
+        for y in (0, 2000003, dims.ny - 1):
+            g.add_source_values(4, y, 3, 2, np.linspace(1.0, 2.0, steps).astype(np.float32))
+            g.add_probe_tables(5, y, 4, 0, np.zeros((steps, 0)), np.zeros((steps, 0)), 0, True)
+            g.add_probe_tables(4, y, 3, 2, np.zeros((steps, 0)), np.zeros((steps, 0)), 0, True)
+
+    def traces(g):
+        return [g.probe_trace(k, steps) for k in range(6)]
+
+    try:
+        out = {}
+        for kernel in ("auto", "fused", "split"):
+            with wf.DeviceFieldGrid(dims, kernel=kernel) as g:
+                t = wf.MaterialTable.vacuum_filled(configs.courant_dt(1e-3), 1e-3)
+                g.set_scene("", t, configs.courant_dt(1e-3), 1e-3)
+                with pytest.raises(wf.WfError):
+                    g.set_tiling(*BRICK)
+                load(g)
+                g.step(steps)
+                g.sync()
+                out[kernel] = traces(g)
+        with wf.DeviceBatch([dims]) as b:
+            assert b.tiling() == (4, 16, 3)
+            b.grid(0).set_scene("", wf.MaterialTable.vacuum_filled(configs.courant_dt(1e-3), 1e-3),
+                                configs.courant_dt(1e-3), 1e-3)
+            load(b.grid(0))
+            b.step(steps)
+            b.sync()
+            out["batch"] = traces(b.grid(0))
+        assert all(np.abs(t).max() > 0 for t in out["split"])
+        for form in ("auto", "fused", "batch"):
+            _same(out[form], out["split"])
+    finally:
+        wf.lib().wf_release_cached_memory(-1)

@@ -51,7 +51,6 @@ namespace {
 constexpr int kBrickMain = kBrickX / 4 * kBrickY * kBrickZ;
 constexpr int kYh = 8 * kBrickZ, kZh = kYh + 64, kXh = kZh + 8 * kBrickZ;
 constexpr int kBrickThreads = kBrickMain + kXh;
-constexpr int kBrickBand = 8;  // rows of bricks per sweep of z (see k_brick)
 
 template <typename ST>
 struct BrickL {

@@ -358,7 +358,9 @@ bool brick_ok(const wf_handle *h) {
   if (h->kernel_pref == WF_KERNEL_SPLIT || encode_fn() == nullptr) return false;
   if (store16(h) && !marching_ok(h)) return false;
   const long long ids = static_cast<long long>(h->mat_pitch) * h->ny * h->nz;
-  return ids < (1ll << 31) && h->nx <= (1 << 19) && h->nz <= (1 << 17);
+  constexpr int kGridZ = 65535;  // bands of rows: the launch's z extent
+  return ids < (1ll << 31) && h->nx <= (1 << 19) && h->nz <= (1 << 17) &&
+         h->ny <= kGridZ * wf::kBrickBand * wf::kBrickY;
 }
 
 // The tiling that names the brick step.
@@ -1092,13 +1094,17 @@ int narrow_item_class(const FusedArgs &a, int k) {
 }
 
 // (Re)builds the batch's device tables when any grid's tables changed.
-// The tiling a batch runs: the caller's, or the cheaper of bricks and marching
-// items (wf_price.h).
+// The tiling a batch runs: the caller's, or the cheaper of bricks (where every
+// grid's can be launched) and marching items (wf_price.h).
 FusedConfig batch_cfg(const wf_batch *b) {
   if (b->cfg_user_set) return b->cfg;
   std::vector<wf::StepShape> shapes;
-  for (const wf_handle *h : b->h) shapes.push_back(step_shape(h));
-  if (wf::batch_takes_bricks(shapes.data(), static_cast<int>(shapes.size())))
+  bool fit = true;
+  for (const wf_handle *h : b->h) {
+    shapes.push_back(step_shape(h));
+    fit = fit && brick_ok(h);
+  }
+  if (fit && wf::batch_takes_bricks(shapes.data(), static_cast<int>(shapes.size())))
     return FusedConfig{wf::kBrickY, wf::kBrickZ, 1};
   return FusedConfig{4, wf::price::kBatchChunk, 3};
 }

@@ -47,6 +47,7 @@ struct FusedArgs {
 
 // Brick step (wf_brick_impl.cuh): one CTA per brick of cells.
 constexpr int kBrickX = 32, kBrickY = 8, kBrickZ = 4;
+constexpr int kBrickBand = 8;  // rows of bricks per sweep of z (see k_brick)
 
 // Sources and probes a brick step applies itself (on = 0: none, or a k_tail
 // launch follows): at most 32 of each.  step: the index of this step, read;
