@@ -205,3 +205,21 @@ def test_scene_voxelizer_bit_identical_to_oracle(oracle):
     g = wf.MaterialGrid(wf.GridDims(64, 64, 64))
     wf.demo_sphere(g)
     assert np.array_equal(g.ids, oracle.demo_sphere(64, 64, 64))
+
+
+def test_axis_profiles_hold_a_value_per_cell_the_library_reads():
+    """wf_set_pml reads n values of each profile: shorter ones are spread from
+    the graded cells' values or refused, never read past their end."""
+    from wavefront_b200.engine import axis_profile
+    full = np.arange(40, dtype=np.float64)
+    assert np.array_equal(axis_profile(full, 40, 7, 1.0), full) and axis_profile(full, 40, 7, 1.0).dtype == np.float32
+    assert len(axis_profile(full, 24, 7, 1.0)) == 40  # longer ones stay: the first n are read
+    got = axis_profile(np.arange(1, 15), 40, 7, 0.5)
+    assert np.array_equal(got[:7], np.arange(1, 8)) and np.array_equal(got[33:], np.arange(8, 15))
+    assert (got[7:33] == 0.5).all() and len(got) == 40
+    for bad in (0, 1, 13, 15, 39):
+        with pytest.raises(ValueError, match="CPML profile"):
+            axis_profile(np.ones(bad), 40, 7, 1.0)
+    with pytest.raises(ValueError, match="CPML profile"):  # slabs that meet need every cell
+        axis_profile(np.ones(30), 40, 25, 1.0)
+    assert len(axis_profile(np.ones(3), 40, 0, 1.0)) == 3  # no layer: nothing is read

@@ -32,6 +32,24 @@ PSI_NAMES = ["psi_ez_dx", "psi_ey_dx", "psi_ez_dy", "psi_ex_dy", "psi_ey_dz", "p
              "psi_hz_dx", "psi_hy_dx", "psi_hx_dy", "psi_hz_dy", "psi_hy_dz", "psi_hx_dz"]
 
 
+def axis_profile(values, n: int, thickness: int, inner: float) -> np.ndarray:
+    """A CPML profile of an axis of n cells as the library reads it: float32, at
+    least n values.  One value per graded cell, min(2 * thickness, n) in all, is
+    spread over the axis with `inner` between the ends; any other shorter length
+    is an error."""
+    v = np.ascontiguousarray(values, np.float32).reshape(-1)
+    if not 0 < thickness <= n or len(v) >= n:  # no layer or a bad one: the library decides
+        return v
+    w = min(2 * thickness, n)
+    if len(v) != w:
+        raise ValueError(f"CPML profile of {len(v)} values: an axis of {n} cells with {thickness} graded "
+                         f"at each end needs {n}, or {w} at the graded cells")
+    out = np.full(n, inner, np.float32)
+    out[:thickness] = v[:thickness]
+    out[n - w + thickness:] = v[thickness:]
+    return out
+
+
 class DeviceFieldGrid:
     def __init__(self, dims: GridDims, boundary=("zero", "zero", "zero"), arith: str = "exact",
                  kernel: str = "auto", device: int = 0, stream: Optional[int] = None,
@@ -125,12 +143,14 @@ class DeviceFieldGrid:
     def set_pml(self, ctx: PmlContext):
         for axis in range(3):
             p = ctx.profiles[axis]
-            t = ctx.thickness_voxels[axis]
-            self._chk(_L.lib().wf_set_pml(self._h, axis, t, _L.ptr(p.b, _L.f32p),
-                                          _L.ptr(p.a, _L.f32p), _L.ptr(p.inv_kappa, _L.f32p)))
+            self.set_pml_axis(axis, ctx.thickness_voxels[axis], p.b, p.a, p.inv_kappa)
 
     def set_pml_axis(self, axis: int, thickness: int, b, a, inv_kappa):
-        b, a, k = (np.ascontiguousarray(v, np.float32) for v in (b, a, inv_kappa))
+        """CPML of `thickness` cells at each end of an axis.  Each profile holds
+        a value per cell of the axis, or one per graded cell (the low end's, then
+        the high end's)."""
+        n = (self.dims.nx, self.dims.ny, self.dims.nz)[axis]
+        b, a, k = (axis_profile(v, n, thickness, inner) for v, inner in ((b, 1.0), (a, 0.0), (inv_kappa, 1.0)))
         self._chk(_L.lib().wf_set_pml(self._h, axis, thickness, _L.ptr(b, _L.f32p),
                                       _L.ptr(a, _L.f32p), _L.ptr(k, _L.f32p)))
 
