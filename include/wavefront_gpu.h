@@ -321,7 +321,8 @@ wf_status wf_get_tiling(const wf_handle *h, wf_tiling *out);
 wf_status wf_set_tiling(wf_handle *h, const wf_tiling *t);
 /* Times each candidate tiling for `steps` steps, and the default step where
  * no tiling names it, and keeps the fastest (`best`: as wf_get_tiling reports
- * it).  After wf_set_column_tiles the candidates are z-marches. */
+ * it).  After wf_set_column_tiles chose the z-march the candidates are
+ * z-marches. */
 wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms);
 /* Fused-kernel work layout of the x-CPML slabs (no counterpart in the
  * reference, whose rayon slabs split along z only, src/engine.rs:291-422).
@@ -330,8 +331,9 @@ wf_status wf_autotune(wf_handle *h, int steps, wf_tiling *best, float *best_ms);
  * 128-cell tiles cover x in [16, nx-16) with no x-psi work; this applies when
  * the x CPML is at most 16 cells deep and nx >= 48.  Off: the wide tiles
  * cover the whole x range and their edge lanes run the x-psi recursion.
- * Either call selects the z-march over the brick step, which has no column
- * tiles, unless a tiling was set.
+ * Off selects the z-march over the brick step, which has no column tiles,
+ * unless a tiling was set; so does on with kernel FUSED.  On with kernel AUTO
+ * is the default: the automatic step, whose z-march, where it runs, has them.
  * Results are bit-identical either way. */
 wf_status wf_set_column_tiles(wf_handle *h, int enable);
 /* 1 when the handle's fused step uses column tiles, 0 otherwise, -1 on a

@@ -275,3 +275,21 @@ def test_grids_beyond_a_brick_launch_run_other_forms():
             _same(out[form], out["split"])
     finally:
         wf.lib().wf_release_cached_memory(-1)
+
+
+def test_asking_for_the_default_column_tiles_leaves_a_grid_automatic():
+    dims = wf.GridDims(64, 64, 64)
+    for kernel, enable, tiling, columns in (("auto", True, BRICK, False), ("auto", False, (4, 12, 3), False),
+                                            ("fused", True, (4, 12, 3), True), ("fused", False, (4, 12, 3), False)):
+        with wf.DeviceFieldGrid(dims, kernel=kernel) as g:
+            p = wf.PmlProfile1D.build(64, wf.PmlConfig(thickness=8), 1e-12, 1e-3, 8)
+            for ax in range(3):
+                g.set_pml_axis(ax, 8, p.b, p.a, p.inv_kappa)
+            g.set_column_tiles(enable)
+            assert (g.tiling(), g.column_tiles) == (tiling, columns), (kernel, enable)
+            if kernel == "auto":  # off and on again: automatic
+                g.set_column_tiles(False)
+                g.set_column_tiles(True)
+                assert g.tiling() == BRICK
+            g.step(2)
+            g.sync()

@@ -115,7 +115,7 @@ struct wf_handle {
   FusedConfig cfg{4, 12, 3};
   int test_extra_tx = 0;      // wf_set_test_stall
   bool cfg_user_set = false;  // otherwise chosen from the grid at first use
-  bool col_user_set = false;  // wf_set_column_tiles was called
+  bool col_user_set = false;  // wf_set_column_tiles asked for a z-march
   wf::StepForm form = wf::StepForm::kSplit;  // of the step (set with the maps)
   wf::InteriorBox mix{};                      // kMix: the marching tiles' box
   wf::BrickMaps brick_map[2];  // per state buffer read
@@ -2119,7 +2119,9 @@ wf_status wf_set_column_tiles(wf_handle *h, int enable) {
   WF_CUDA(h, cudaStreamSynchronize(h->stream));
   drop_graphs(h);
   h->col_pref = enable != 0;
-  h->col_user_set = true;
+  // asking an automatic grid for the default changes nothing; kernel=fused asks
+  // for the z-march either way
+  h->col_user_set = !enable || h->kernel_pref == WF_KERNEL_FUSED;
   ++h->version;
   h->maps_ok = false;
   return WF_OK;
