@@ -143,3 +143,74 @@ def test_device_memory_cache_reuses_and_releases():
         g.close()
     assert lib.wf_release_cached_memory(-1) == L.WF_OK
     assert lib.wf_cached_bytes(0) == 0
+
+
+def _stalled_step(g, load, limit):
+    """One normal step, then one whose copies never complete: WF_ERR_TIMEOUT
+    within `limit` seconds; returns the seconds it took."""
+    load(g)
+    g.step(1)
+    g.sync()
+    g.set_test_stall(16)
+    t0 = time.perf_counter()
+    g.step(1)
+    with pytest.raises(wf.WfError) as e:
+        g.sync()
+    waited = time.perf_counter() - t0
+    assert e.value.status == L.WF_ERR_TIMEOUT
+    assert 0.3 < waited < limit, waited
+    return waited
+
+
+@pytest.mark.parametrize("tiling,columns,precision", [
+    ((8, 4, 1), None, "f32"), ((4, 12, 3), False, "f32"), ((4, 12, 3), True, "f32"), ((8, 4, 1), None, "f16"),
+    ((4, 32, 3), True, "f16")])
+def test_stalled_stage_in_every_form_of_the_step(tiling, columns, precision):
+    """Bricks, the marching tiles and their column tiles each report a wait
+    that ran out, and the grid's next step after the stall is taken off is a
+    step like any other on a new handle."""
+    sc = configs.plain_cube_64(steps=4)
+    g = configs.device_grid(sc, precision=precision)
+    try:
+        g.set_tiling(*tiling)
+        if columns is not None:
+            g.set_column_tiles(columns)
+            assert g.column_tiles == columns
+        _stalled_step(g, lambda h: _configure(h, sc, 4), 60.0)
+    finally:
+        g.close()
+    with configs.device_grid(sc) as h:
+        _configure(h, sc, 4)
+        h.step(4)
+        h.sync()
+        assert np.isfinite(h.fields()).all()
+
+
+def test_a_stalled_step_of_many_bricks_ends_soon():
+    """256^3 with CPML is some 55 waves of bricks: one wait of about a second
+    in all, not two a wave."""
+    n, t = 256, 8
+    g = wf.DeviceFieldGrid(wf.GridDims(n, n, n))
+    try:
+        p = wf.PmlProfile1D.build(n, wf.PmlConfig(thickness=t), 1e-12, 1e-3, t)
+        for ax in range(3):
+            g.set_pml_axis(ax, t, p.b, p.a, p.inv_kappa)
+        g.set_tiling(8, 4, 1)
+        print("stalled step of 256^3 bricks:", _stalled_step(g, lambda h: None, 10.0), "s")
+    finally:
+        g.close()
+
+
+def test_a_stalled_grid_of_a_batch_is_reported():
+    scenes = configs.batched_sweep(2, steps=4, seed=41, sizes=(32,))
+    b = configs.device_batch(scenes)
+    try:
+        b.set_tiling(8, 4, 1)
+        b.grid(1).set_test_stall(16)
+        t0 = time.perf_counter()
+        b.step(1)
+        with pytest.raises(wf.WfError) as e:
+            b.sync()
+        assert e.value.status == L.WF_ERR_TIMEOUT and time.perf_counter() - t0 < 20.0
+    finally:
+        b.close()

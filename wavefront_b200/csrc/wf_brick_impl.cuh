@@ -530,15 +530,16 @@ __device__ __forceinline__ void brick_body(const CUtensorMap *tmE, const CUtenso
   }
 
   __syncthreads();  // the mbarrier is initialised
-  bool ok = mbar_wait(smem_u32(&s_bar), 0);
+  bool ok = mbar_wait_or_error(smem_u32(&s_bar), 0, g.err);
   ok = __syncthreads_or(ok ? 0 : 1) == 0;
   if (!ok) {
     // the phase never completed within the limit: latch the error (without an
     // error word, the caller's own fields: the brick's new values become NaN);
-    // one more bounded wait before this CTA's shared memory is released
+    // one more bounded wait before this CTA's shared memory is released (short
+    // when the error is latched: its copies have had the first wait)
     if (tid == 0) {
       if (g.err) atomicOr(g.err, kErrTimeout);
-      mbar_wait(smem_u32(&s_bar), 0);
+      mbar_wait_or_error(smem_u32(&s_bar), 0, g.err);
     }
     if (!g.err && role == 0 && in) {
       if constexpr (!U)

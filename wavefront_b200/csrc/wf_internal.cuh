@@ -19,6 +19,7 @@ namespace wf {
 
 constexpr int kTileX = 128;          // cells per tile row: 32 lanes x float4
 constexpr long long kWaitLimitCycles = 2000000000LL;  // ~1 s at B200 clocks
+constexpr long long kWaitAfterErrorCycles = 2000000LL;  // ~1 ms: see mbar_wait_or_error
 
 // Device error bits (latched in a device word, reported by wf_sync).
 enum : int { kErrTimeout = 1, kErrBounds = 2 };
@@ -171,6 +172,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity)) {
     if (clock64() - t0 > kWaitLimitCycles) return false;
+  }
+  return true;
+}
+
+// The same in launches of many short CTAs, whose waits would add up wave by
+// wave: once the error word says that some wait has run out, a wait that has
+// lasted a thousand times a copy's usual time gives up too.  512^3 in bricks is
+// some 300 waves: about 1.5 s for a step whose copies never land, not minutes.
+__device__ __forceinline__ bool mbar_wait_or_error(uint32_t bar, uint32_t parity, const int *err) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    const long long t = clock64() - t0;
+    if (t > kWaitLimitCycles) return false;
+    if (t > kWaitAfterErrorCycles && err && (*reinterpret_cast<const volatile int *>(err) & kErrTimeout))
+      return false;
   }
   return true;
 }
