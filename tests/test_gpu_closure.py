@@ -392,3 +392,12 @@ def test_convolutions_of_several_widths_from_several_threads():
     assert not bad, bad
     for d, w in zip(data, want):
         assert torch.equal(d[2], w)
+
+
+@pytest.mark.parametrize("n,ci,co,d,h,w,nface", [
+    (1, 16, 16, 1, 8, 8, 6), (63, 3, 5, 2, 8, 8, 8), (5, 10, 6, 1, 1, 7, 3), (7, 16, 16, 1, 8, 16, 6),
+    (7, 16, 16, 3, 1, 43, 6), (64, 16, 16, 1, 8, 8, 6), (9, 1, 2, 5, 5, 5, 2)])
+def test_weight_gradient_of_samples_of_few_voxels(n, ci, co, d, h, w, nface):
+    """Either side of the sizes where a thread per weight takes over from the
+    tiles (128 voxels, 64 samples); tolerance as above."""
+    test_weight_gradient_against_float64(n, ci, co, d, h, w, nface)

@@ -212,7 +212,32 @@ __device__ float bw_checked(const float *v, const float *g, int t, int d0, int d
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 
 // dw[face][co][ci][tap] += sum over samples of that face and voxels p of
-// dz[n][co][p] * in[n][ci][p + tap].
+// dz[n][co][p] * in[n][ci][p + tap], for samples of few voxels: one thread per
+// weight, the samples split over blockIdx.y, both operands from global memory.
+// The tiles below cost 16 to 18 us however little there is to sum (their
+// unrolled code is fetched once and run once): 1 sample of 8 x 8, 16 -> 16
+// channels, takes 11.6 us here and 17.8 there, 63 of 4 x 4 15 and 32; at 128
+// voxels a sample the two are equal.
+constexpr int kBwFewVoxels = 128;
+__global__ void k_conv_bwd_weight_few(const float *in, const float *dz, const int *face, float *dw, int n,
+                                      int ci, int co, int D, int H, int W, int nface) {
+  const int nw = co * ci * kTaps, e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nw) return;
+  const int o = e / (ci * kTaps), c = (e / kTaps) % ci, t = e % kTaps;
+  const long long P = static_cast<long long>(D) * H * W;
+  float acc[8];  // by face
+  for (float &a : acc) a = 0.0f;
+  for (int s = blockIdx.y; s < n; s += gridDim.y) {
+    const int f = face ? face[s] : 0;
+    if (f < 0 || f >= nface) continue;
+    acc[f] += bw_checked(in + (static_cast<long long>(s) * ci + c) * P, dz + (static_cast<long long>(s) * co + o) * P,
+                         t, 0, D, 0, H, 0, W, D, H, W, 0.0f);
+  }
+  for (int f = 0; f < nface; ++f)
+    if (acc[f] != 0.0f) atomicAdd(dw + static_cast<long long>(f) * nw + e, acc[f]);
+}
+
+// The same from tiles in shared memory.
 //
 // A CTA works for one face (blockIdx.y) on every gridDim.x-th tile of the
 // face's samples: 4 planes x 4 rows x 16 columns of dz and their haloed input
@@ -290,11 +315,13 @@ __global__ void __launch_bounds__(kBwThreads, 2)
         }
         __syncthreads();
         if (!active) continue;
+        const int xe = min(kBwX, W - x0);  // rows and columns of padding add zeros: left out
         for (int row = part; row < kBwD * kBwY; row += parts) {
+          if (d0 + row / kBwY >= D || y0 + row % kBwY >= H) continue;
           const float *z0 = s_dz + o * kBwDz + row * kBwX;
           const float *v = s_in + c * kBwIn + (row / kBwY * (kBwY + 2) + row % kBwY) * kBwRow;
 #pragma unroll 1
-          for (int x = 0; x < kBwX; x += 4) {
+          for (int x = 0; x < xe; x += 4) {
             const float4 ga = *reinterpret_cast<const float4 *>(z0 + x);
             const float4 gb = *reinterpret_cast<const float4 *>(z0 + kBwDz + x);
             const float g0[4] = {ga.x, ga.y, ga.z, ga.w}, g1[4] = {gb.x, gb.y, gb.z, gb.w};
@@ -787,6 +814,11 @@ int nn_conv_bwd_weight(const float *in, const float *dz, const int *face, float 
   if (ci < 1 || co < 1) return cudaErrorInvalidConfiguration;  // as an empty launch grid
   if (nface < 1 || D < 1 || H < 1 || W < 1) return cudaSuccess;  // nothing to add
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (n < 64 && static_cast<long long>(D) * H * W <= kBwFewVoxels) {
+    const dim3 grid(blocks_for(co * ci * kTaps, 128), std::min(n, 64));
+    k_conv_bwd_weight_few<<<grid, 128, 0, st>>>(in, dz, face, dw, n, ci, co, D, H, W, nface);
+    return cudaGetLastError();
+  }
   // one CTA per sample where there are enough samples and the planes fit
   const BsGeom G = bs_geom(H, W);
   constexpr int kSmemMax = 227 * 1024;
