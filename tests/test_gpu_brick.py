@@ -293,3 +293,17 @@ def test_asking_for_the_default_column_tiles_leaves_a_grid_automatic():
                 assert g.tiling() == BRICK
             g.step(2)
             g.sync()
+
+
+# The marching tiles, which a grid of these sizes runs only when asked: FMA and
+# exact, every CPML class, column tiles on (the default) and off.
+@pytest.mark.parametrize("tiling", [(4, 12, 3), (8, 16, 3), (16, 5, 3), (4, 24, 4)])
+@pytest.mark.parametrize("dims,pml,kw", [
+    ((136, 72, 40), (10, 10, 10), {"arith": "fma"}),
+    ((136, 72, 40), (16, 0, 12), {"arith": "fma", "nsrc": 33}),
+    ((264, 40, 56), (7, 5, 0), {"arith": "fma", "sheet": True}),
+    ((72, 72, 48), (20, 9, 16), {"arith": "fma"}),
+    ((136, 72, 40), (10, 10, 10), {}),
+])
+def test_marching_equals_split(tiling, dims, pml, kw):
+    _same(_grid(dims, "fused", 43, pml, tiling=tiling, **kw), _grid(dims, "split", 43, pml, **kw))
