@@ -7,10 +7,10 @@
 // partly outside, 0- to 48-cell CPML on any axes, zero and periodic boundaries,
 // exact and FMA, FP32 and 16-bit; fields of noise).  Over those grids the form
 // picked takes 0.2 % more than the best one on average (0.2 % too on a half left
-// out of the fit), 9 of them more than 6 %.  A rule on the cells alone lost up to 1.8x: bricks
-// cost the same with 8 of their 32 columns inside as with all (16 x 256 x 256,
-// periodic: split 24 us, bricks 44), and the interior of a mixed step pays for
-// whole 128-cell tiles.
+// out of the fit), 10 of them more than 6 %.  A rule on the cells alone lost up
+// to 1.8x: bricks cost the same with 8 of their 32 columns inside as with all
+// (16 x 256 x 256, periodic: split 24 us, bricks 44), and the interior of a mixed
+// step pays for whole 128-cell tiles.
 //
 // Host code without CUDA types: compiles on its own.
 #pragma once
@@ -250,7 +250,9 @@ inline bool interior_box(const StepShape &s, InteriorBox *m) {
 // The split pair is charged 12 % where marching tiles could run: its fit is
 // that far off on short rows with slabs, and bricks lose little there.  With
 // CPML on x alone marching tiles are charged 5 %: their fit is up to 9 % low on
-// 16-cell slabs there (512^3: 1408 us, bricks around them 1368).
+// 16-cell slabs there (512^3: 1408 us, bricks around them 1368).  The mixed step
+// has to be 3.5 % below bricks: its work lists, streams and graphs with forks cost
+// a new grid more (256^3 with 8 cells, its first 50 steps: 14.3 ms, bricks 11.9).
 inline StepForm cheapest_step(const StepShape &s, bool march_ok, bool brick_ok, bool split_ok) {
   const bool pml = price::has_cpml(s), x_alone = s.depth[0] > 0 && !(s.depth[1] | s.depth[2]);
   StepForm best = StepForm::kSplit;
@@ -264,10 +266,13 @@ inline StepForm cheapest_step(const StepShape &s, bool march_ok, bool brick_ok, 
   InteriorBox box;
   if (march_ok) offer(StepForm::kMarch, price::march_us(s) * (x_alone ? 1.05 : 1.0));
   if (split_ok && !s.b16) offer(StepForm::kSplit, price::split_us(s) * (march_ok ? 1.12 : 1.0));
-  if (brick_ok)
-    offer(StepForm::kBrick,
-          price::brick_us(s) * (pml ? 1.0 : (s.b16 ? 1.10 : (price::any_periodic(s) ? 1.03 : 1.05))));
-  if (march_ok && brick_ok && interior_box(s, &box)) offer(StepForm::kMix, price::mix_us(s, box));
+  if (!brick_ok) return best;
+  const double bricks = price::brick_us(s);
+  offer(StepForm::kBrick, bricks * (pml ? 1.0 : (s.b16 ? 1.10 : (price::any_periodic(s) ? 1.03 : 1.05))));
+  if (march_ok && interior_box(s, &box)) {
+    const double mix = price::mix_us(s, box);
+    if (mix * 1.035 < bricks) offer(StepForm::kMix, mix);
+  }
   return best;
 }
 
