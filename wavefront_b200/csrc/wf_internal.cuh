@@ -179,7 +179,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 // The same in launches of many short CTAs, whose waits would add up wave by
 // wave: once the error word says that some wait has run out, a wait that has
 // lasted a thousand times a copy's usual time gives up too.  512^3 in bricks is
-// some 300 waves: about 1.5 s for a step whose copies never land, not minutes.
+// some 440 waves: about 1.5 s for a step whose copies never land, not minutes.
 __device__ __forceinline__ bool mbar_wait_or_error(uint32_t bar, uint32_t parity, const int *err) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
