@@ -315,9 +315,10 @@ __global__ void __launch_bounds__(kBwThreads, 2)
         }
         __syncthreads();
         if (!active) continue;
-        const int xe = min(kBwX, W - x0);  // rows and columns of padding add zeros: left out
-        for (int row = part; row < kBwD * kBwY; row += parts) {
-          if (d0 + row / kBwY >= D || y0 + row % kBwY >= H) continue;
+        // rows and columns of padding add zeros: left out
+        const int xe = min(kBwX, W - x0), ye = min(kBwY, H - y0), rows = min(kBwD, D - d0) * kBwY;
+        for (int row = part; row < rows; row += parts) {
+          if (row % kBwY >= ye) continue;
           const float *z0 = s_dz + o * kBwDz + row * kBwX;
           const float *v = s_in + c * kBwIn + (row / kBwY * (kBwY + 2) + row % kBwY) * kBwRow;
 #pragma unroll 1
