@@ -12,6 +12,7 @@ src/probe.rs:127).  Fields, every probe's sums and counts are compared.
 import numpy as np
 import pytest
 
+import wavefront_b200 as wf
 from wavefront_b200 import configs
 from wavefront_b200.probe import FieldComponent as PC
 from wavefront_b200.probe import Probe
@@ -75,3 +76,48 @@ def test_sources_and_probes_added_between_steps(kernel):
     finally:
         early.close()
         late.close()
+
+
+@pytest.mark.parametrize("form", ["fused", "split", "batch"])
+def test_first_sources_and_probes_after_steps_without_any(form):
+    """A source's values and a probe's tables count from the handle's first
+    step, also where no step before had a source or probe: 7 bare steps, then
+    both, equal a grid that had them, silent until then, from the start."""
+    bare, rest = 7, 40
+    steps = bare + rest
+    sc = configs.plain_cube_64(steps=steps)
+    f0 = sc.meta["f0"]
+    s2 = Source(20, 40, 28, FieldComponent.Ey, 0.5, default_waveform("gaussian", f0))
+    p2 = Probe(22, 39, 30, PC.Hz, [f0, 0.5 * f0], 0.0)
+    v = s2.values(sc.dt, steps)
+    silent = v.copy()
+    silent[:bare] = 0.0
+    assert np.abs(v[:bare]).max() > 0 and not np.array_equal(v[:rest], v[bare:])
+    c, si = p2.tables(sc.dt, steps)
+    f = np.random.default_rng(5).standard_normal((6, 64, 64, 64)).astype(np.float32)
+
+    def run(late):
+        if form == "batch":
+            b = wf.DeviceBatch([sc.dims, sc.dims])
+            grids, step, close = b.grids, b.step, b.close
+            for g in grids:
+                g.set_materials(sc.grid, sc.table)
+        else:
+            g = configs.device_grid(sc, kernel=form)
+            grids, step, close = [g], g.step, g.close
+        g = grids[0]
+        try:
+            g.set_fields(f)
+            if late:
+                step(bare)
+            g.add_source_values(s2.x, s2.y, s2.z, s2.component, v if late else silent)
+            g.add_probe_tables(p2.x, p2.y, p2.z, p2.component, c, si, bare, True)
+            step(steps - bare if late else steps)
+            g.sync()
+            sums = g.probe_sums(0, 2)
+            return [g.fields(), sums[0], sums[1], np.array(sums[2]), g.probe_trace(0, steps)[bare:]]
+        finally:
+            close()
+
+    for name, got, want in zip(("fields", "cos", "sin", "count", "trace"), run(True), run(False)):
+        _eq(got, want, name)

@@ -922,6 +922,10 @@ wf_status upload_src_probe_tables(wf_handle *h) {
     WF_CUDA(h, wf::dev_alloc(&h->d_probe, sizeof(ProbeDev) * v.size()));
     WF_CUDA(h, h2d_sync(h->d_probe, v.data(), sizeof(ProbeDev) * v.size(), h->stream));
   }
+  // steps without sources and probes do not count on the device: values and
+  // tables are indexed from the handle's first step all the same
+  const long long step[2] = {h->steps_done, h->steps_done};
+  WF_CUDA(h, h2d_sync(h->d_step, step, sizeof(step), h->stream));
   return WF_OK;
 }
 
